@@ -6,10 +6,11 @@
 #include <stdint.h>
 
 #include <algorithm>
-
+#include <atomic>
 #include <mutex>
 
 #include "ivr_internal.h"
+#include "ivr_mlp.h"
 
 namespace ivr {
 namespace {
@@ -62,14 +63,104 @@ __global__ void gather_kernel(const T *__restrict__ src, int gw, int gh, T *__re
     }
 }
 
-__global__ void minmax_kernel(const void *data, int dtype, long long n, float *partial)
+// 16 bytes of voxels at a time: the passes over a whole volume (min/max,
+// histogram) read it with aligned vector loads; the volume's own array is a
+// device allocation, so its base is aligned for every dtype, and the last
+// n % kVec voxels are read one by one.
+template <typename T> constexpr int kVec = 16 / (int) sizeof(T);
+
+template <typename T> __device__ __forceinline__ T vox_of(const uint4 &q, int e)
 {
+    const unsigned w = (&q.x)[e * (int) sizeof(T) / 4];
+    if constexpr (sizeof(T) == 4) return __uint_as_float(w);
+    else return (T) (w >> (8 * ((e * (int) sizeof(T)) & 3)));
+}
+
+// Min and max of the volume, one pair per block.  Bound by HBM.  Each thread
+// keeps four 16-byte loads in flight; integer voxels are compared as packed
+// lanes and converted once at the end (the conversion is exact and
+// monotone), floats with fminf/fmaxf, which pass over NaNs.
+template <typename T> struct MinMaxAcc {
+    // packed lanes of a 32-bit word
+    unsigned lo = 0xffffffffu, hi = 0u;
+    __device__ __forceinline__ void word(unsigned w)
+    {
+        if constexpr (sizeof(T) == 1) {
+            lo = __vminu4(lo, w);
+            hi = __vmaxu4(hi, w);
+        } else {
+            lo = __vminu2(lo, w);
+            hi = __vmaxu2(hi, w);
+        }
+    }
+    __device__ __forceinline__ void one(T v)
+    {
+        unsigned w = v;
+        for (int b = 8 * (int) sizeof(T); b < 32; b *= 2) w |= w << b;
+        word(w);
+    }
+    __device__ __forceinline__ void get(float &l, float &h) const
+    {
+        unsigned a = 0xffffffffu, b = 0u;
+        for (int e = 0; e < 4 / (int) sizeof(T); e++) {
+            a = min(a, (unsigned) (T) (lo >> (8 * (int) sizeof(T) * e)));
+            b = max(b, (unsigned) (T) (hi >> (8 * (int) sizeof(T) * e)));
+        }
+        l = (float) a;
+        h = (float) b;
+    }
+};
+template <> struct MinMaxAcc<float> {
     float lo = FLT_MAX, hi = -FLT_MAX;
-    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
-        float v = load_any(data, dtype, i);
+    __device__ __forceinline__ void one(float v)
+    {
         lo = fminf(lo, v);
         hi = fmaxf(hi, v);
     }
+    __device__ __forceinline__ void word(unsigned w) { one(__uint_as_float(w)); }
+    __device__ __forceinline__ void get(float &l, float &h) const
+    {
+        l = lo;
+        h = hi;
+    }
+};
+
+template <typename T>
+__global__ void minmax_kernel(const T *__restrict__ data, long long n, float *partial)
+{
+    MinMaxAcc<T> acc;
+    const long long nv = n / kVec<T>, stride = (long long) gridDim.x * blockDim.x;
+    const long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
+    const uint4 *q = reinterpret_cast<const uint4 *>(data);
+    long long i = t;
+    bool any = false;
+    for (; i + 3 * stride < nv; i += 4 * stride) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = __ldcs(q + i + u * stride);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            acc.word(v[u].x);
+            acc.word(v[u].y);
+            acc.word(v[u].z);
+            acc.word(v[u].w);
+        }
+        any = true;
+    }
+    for (; i < nv; i += stride) {
+        const uint4 v = __ldcs(q + i);
+        acc.word(v.x);
+        acc.word(v.y);
+        acc.word(v.z);
+        acc.word(v.w);
+        any = true;
+    }
+    if (t < n - nv * kVec<T>) {
+        acc.one(__ldg(data + nv * kVec<T> + t));
+        any = true;
+    }
+    float lo = FLT_MAX, hi = -FLT_MAX;
+    if (any) acc.get(lo, hi);
     for (int o = 16; o > 0; o >>= 1) {
         lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
         hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
@@ -85,28 +176,101 @@ __global__ void minmax_kernel(const void *data, int dtype, long long n, float *p
     }
 }
 
-// histogram (mathutil.c:459-467): bin (int)(v - min); privatised in shared
-// memory when the bins fit.
-constexpr int kSmemBins = 12288;
-__global__ void hist_smem_kernel(const void *data, int dtype, long long n, float mn, int hsize, int *hist)
+// The value range as a kernel argument: known to the host, or still in
+// device memory (the allocation-free histogram).
+struct MinArg {
+    float v;
+    const float *dev;
+};
+
+// histogram (mathutil.c:459-467): bin (int)(v - min).  Bound by the atomics:
+// one shared-memory counter per voxel, and background voxels that all want
+// the same one.  (One global atomic per voxel above 12,288 bins took 65.7 ms
+// for 512^3 u16 voxels with 70% background; with its result copied to the
+// host this takes 0.22 ms.)
+// - The bins are cut into `gridDim.y` ranges of `nb` that fit a block's
+//   shared memory (65,536 bins take two ranges of 128 KB: 256 KB do not fit
+//   an SM); every range's blocks read the whole volume, the second reader
+//   mostly from L2.
+// - A range with room to spare keeps 2^rep copies of each counter, the copy
+//   by lane, so that equal neighbours in a warp do not wait for each other.
+// - Each thread counts bin 0 (the minimum: the background) in a register and
+//   runs of one bin as one addition.
+template <typename T>
+__global__ void __launch_bounds__(1024) hist_kernel(const T *__restrict__ data, long long n, MinArg mn, int hsize,
+                                                    int nb, int rep, int *hist)
 {
-    __shared__ int sh[kSmemBins];
-    for (int b = threadIdx.x; b < hsize; b += blockDim.x) sh[b] = 0;
+    extern __shared__ int sh[];
+    const int first = (int) blockIdx.y * nb, bins = min(nb, hsize - first);
+    for (int b = threadIdx.x; b < bins << rep; b += blockDim.x) sh[b] = 0;
     __syncthreads();
-    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
-        int b = (int) (load_any(data, dtype, i) - mn);
-        if (b >= 0 && b < hsize) atomicAdd(&sh[b], 1);
+    const float fmin = mn.dev ? __ldg(mn.dev) : mn.v;
+    // integer voxels: their minimum is an integer too, and the float
+    // difference the rule takes is exact, so the bin is the integer difference
+    const int imin = sizeof(T) < 4 ? (int) fmin : 0;
+    const int copy = threadIdx.x & ((1 << rep) - 1);
+    int zero = 0, cur = -1, run = 0;
+    auto add = [&](T v) {
+        const int b = (int) ((unsigned) (sizeof(T) < 4 ? (int) v - imin : (int) ((float) v - fmin)) - (unsigned) first);
+        if (b == 0) {
+            zero++;
+        } else {
+            if (b != cur) {
+                if ((unsigned) cur < (unsigned) bins) atomicAdd(&sh[(cur << rep) + copy], run);
+                cur = b;
+                run = 0;
+            }
+            run++;
+        }
+    };
+    const long long nv = n / kVec<T>, stride = (long long) gridDim.x * blockDim.x;
+    const long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
+    const uint4 *q = reinterpret_cast<const uint4 *>(data);
+    long long i = t;
+    for (; i + stride < nv; i += 2 * stride) {
+        const uint4 v0 = __ldg(q + i), v1 = __ldg(q + i + stride);
+#pragma unroll
+        for (int e = 0; e < kVec<T>; e++) add(vox_of<T>(v0, e));
+#pragma unroll
+        for (int e = 0; e < kVec<T>; e++) add(vox_of<T>(v1, e));
     }
+    for (; i < nv; i += stride) {
+        const uint4 v = __ldg(q + i);
+#pragma unroll
+        for (int e = 0; e < kVec<T>; e++) add(vox_of<T>(v, e));
+    }
+    if (t < n - nv * kVec<T>) add(__ldg(data + nv * kVec<T> + t));
+    if ((unsigned) cur < (unsigned) bins) atomicAdd(&sh[(cur << rep) + copy], run);
+    zero = __reduce_add_sync(0xffffffffu, zero);
+    if ((threadIdx.x & 31) == 0 && zero) atomicAdd(&sh[0], zero);
     __syncthreads();
-    for (int b = threadIdx.x; b < hsize; b += blockDim.x)
-        if (sh[b]) atomicAdd(&hist[b], sh[b]);
+    // neighbouring blocks start at different bins, so that their additions
+    // to the result do not meet
+    const int turn = (int) ((long long) blockIdx.x * bins / gridDim.x);
+    for (int k = threadIdx.x; k < bins; k += blockDim.x) {
+        const int b = k + turn < bins ? k + turn : k + turn - bins;
+        int c = 0;
+        for (int r = 0; r < 1 << rep; r++) c += sh[(b << rep) + ((r + threadIdx.x) & ((1 << rep) - 1))];
+        if (c) atomicAdd(&hist[first + b], c);
+    }
 }
-__global__ void hist_global_kernel(const void *data, int dtype, long long n, float mn, int hsize, int *hist)
+
+// More bins than four ranges hold (float volumes of a wide range): counters
+// in global memory, runs added at once.
+__global__ void hist_global_kernel(const float *__restrict__ data, long long n, MinArg mn, int hsize, int *hist)
 {
+    const float fmin = mn.dev ? __ldg(mn.dev) : mn.v;
+    int cur = -1, run = 0;
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
-        int b = (int) (load_any(data, dtype, i) - mn);
-        if (b >= 0 && b < hsize) atomicAdd(&hist[b], 1);
+        const int b = (int) (__ldg(data + i) - fmin);
+        if (b != cur) {
+            if ((unsigned) cur < (unsigned) hsize) atomicAdd(&hist[cur], run);
+            cur = b;
+            run = 0;
+        }
+        run++;
     }
+    if ((unsigned) cur < (unsigned) hsize) atomicAdd(&hist[cur], run);
 }
 
 // Macrocell min/max: with edge `cell`, cell (cx,cy,cz) spans voxels
@@ -315,26 +479,56 @@ __global__ void minmax_final_kernel(const float *partial, int nparts, float *min
     }
 }
 
-// the histogram of hist_*_kernel with the minimum read from device memory
-__global__ void hist_devmin_kernel(const void *data, int dtype, long long n, const float *minmax, int hsize,
-                                   int *hist)
+constexpr int kHistBlocks = kSms;           // one block an SM
+constexpr int kHistSmem = 224 * 1024;       // shared memory a block may ask for
+constexpr int kHistBins = kHistSmem / 4;    // counters in it
+constexpr int kHistRanges = 4;              // ranges before the bins move to global memory
+
+template <typename T>
+cudaError_t hist_launch(const T *data, long long n, MinArg mn, int hsize, int *hist, cudaStream_t s)
 {
-    __shared__ int sh[kSmemBins];
-    const float mn = minmax[0];
-    const bool priv = hsize <= kSmemBins;
-    if (priv) {
-        for (int b = threadIdx.x; b < hsize; b += blockDim.x) sh[b] = 0;
-        __syncthreads();
+    static std::atomic<unsigned long long> attr{0};
+    cudaError_t e = set_dynamic_smem_once(hist_kernel<T>, kHistSmem, attr);
+    if (e != cudaSuccess) return e;
+    const int ranges = (hsize + kHistBins - 1) / kHistBins;
+    const int nb = (hsize + ranges - 1) / ranges;
+    int rep = 0;
+    while (rep < 5 && (nb << (rep + 1)) <= kHistBins / 2) rep++;  // 112 KB: two blocks an SM
+    const size_t smem = sizeof(int) * ((size_t) nb << rep);
+    const int per_sm = smem <= kHistSmem / 2 ? 2 : 1;
+    // 8192 voxels a block at least: clearing and adding up the counters costs
+    // about that much
+    const long long most = n / 8192 + 1, wave = (long long) kHistBlocks * per_sm / ranges;
+    const dim3 grid((unsigned) (wave < most ? wave : most), ranges);
+    hist_kernel<T><<<grid, 1024, smem, s>>>(data, n, mn, hsize, nb, rep, hist);
+    return cudaGetLastError();
+}
+
+cudaError_t hist_any(const void *data, int dtype, long long n, MinArg mn, int hsize, int *hist, cudaStream_t s)
+{
+    if ((long long) hsize > (long long) kHistRanges * kHistBins) {
+        // integer voxels have at most 65,536 values: bins above are empty
+        if (dtype == IVR_F32) {
+            hist_global_kernel<<<grid_for(n, 256), 256, 0, s>>>((const float *) data, n, mn, hsize, hist);
+            return cudaGetLastError();
+        }
+        hsize = 65536;
     }
-    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
-        int b = (int) (load_any(data, dtype, i) - mn);
-        if (b >= 0 && b < hsize) atomicAdd(priv ? &sh[b] : &hist[b], 1);
+    switch (dtype) {
+    case IVR_U8: return hist_launch((const uint8_t *) data, n, mn, hsize, hist, s);
+    case IVR_U16: return hist_launch((const uint16_t *) data, n, mn, hsize, hist, s);
+    default: return hist_launch((const float *) data, n, mn, hsize, hist, s);
     }
-    if (priv) {
-        __syncthreads();
-        for (int b = threadIdx.x; b < hsize; b += blockDim.x)
-            if (sh[b]) atomicAdd(&hist[b], sh[b]);
+}
+
+cudaError_t minmax_any(const void *data, int dtype, long long n, float *partial, int nparts, cudaStream_t s)
+{
+    switch (dtype) {
+    case IVR_U8: minmax_kernel<<<nparts, 256, 0, s>>>((const uint8_t *) data, n, partial); break;
+    case IVR_U16: minmax_kernel<<<nparts, 256, 0, s>>>((const uint16_t *) data, n, partial); break;
+    default: minmax_kernel<<<nparts, 256, 0, s>>>((const float *) data, n, partial); break;
     }
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -368,11 +562,10 @@ cudaError_t noalloc_histogram(const void *data, int dtype, long long n, int hsiz
     cudaError_t e = noalloc_scratch(&sc);
     if (e != cudaSuccess) return e;
     const int parts = kSms * 4;
-    minmax_kernel<<<parts, 256, 0, s>>>(data, dtype, n, sc->partial);
+    if ((e = minmax_any(data, dtype, n, sc->partial, parts, s)) != cudaSuccess) return e;
     minmax_final_kernel<<<1, 1024, 0, s>>>(sc->partial, parts, sc->minmax);
     if ((e = cudaMemsetAsync(sc->hist, 0, sizeof(int) * (size_t) hsize, s)) != cudaSuccess) return e;
-    hist_devmin_kernel<<<grid_for(n, 512, 2), 512, 0, s>>>(data, dtype, n, sc->minmax, hsize, sc->hist);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = hist_any(data, dtype, n, MinArg{0.0f, sc->minmax}, hsize, sc->hist, s)) != cudaSuccess) return e;
     if ((e = cudaMemcpyAsync(hist_host, sc->hist, sizeof(int) * (size_t) hsize, cudaMemcpyDeviceToHost, s)) !=
         cudaSuccess)
         return e;
@@ -407,17 +600,14 @@ cudaError_t launch_gather_brick(const void *src, int gw, int gh, int gd, void *d
 
 cudaError_t launch_minmax(const void *data, int dtype, long long n, float *partial, int nparts, cudaStream_t s)
 {
-    minmax_kernel<<<nparts, 256, 0, s>>>(data, dtype, n, partial);
-    return cudaGetLastError();
+    return minmax_any(data, dtype, n, partial, nparts, s);
 }
 
 cudaError_t launch_histogram(const void *data, int dtype, long long n, float mn, int hsize, int *hist, cudaStream_t s)
 {
     cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(int) * (size_t) hsize, s);
     if (e != cudaSuccess) return e;
-    if (hsize <= kSmemBins) hist_smem_kernel<<<grid_for(n, 512, 2), 512, 0, s>>>(data, dtype, n, mn, hsize, hist);
-    else hist_global_kernel<<<grid_for(n, 256), 256, 0, s>>>(data, dtype, n, mn, hsize, hist);
-    return cudaGetLastError();
+    return hist_any(data, dtype, n, MinArg{mn, nullptr}, hsize, hist, s);
 }
 
 cudaError_t launch_macrocells(const void *data, int dtype, int nx, int ny, int nz, int cell, float *mc, int mcx,
