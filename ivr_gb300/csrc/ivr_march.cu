@@ -9,6 +9,7 @@
 #include <float.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "ivr_internal.h"
@@ -19,46 +20,39 @@ namespace {
 constexpr int kBlockX = 16;  // pixels per block: 2x2 warps of 8x4
 constexpr int kBlockY = 8;
 constexpr int kThreads = 128;
-#ifndef IVR_CFG_PAIR
-#define IVR_CFG_PAIR 1  // two CONFIG samples per loop iteration
+// Samples of a ray that one loop iteration takes (K), all their loads in
+// flight before the first is composited, and resident blocks per SM each
+// kernel is compiled for (65,536 / (128 blocks) registers a thread).  A
+// launch is bound by the latency of its longest rays as much as by its
+// throughput, so loads in flight within a thread are worth more than warps
+// beside it.  Measured on GB300 (us a frame at K = 2, 4, 6, 8 with 5 blocks,
+// the start of the sweep K = 2 with 9 blocks): u16 learned 1024^3 at
+// 1920x1080 462, 368, 341, 368 (556); u16 without skipping 266, 218, 198,
+// 200 (368); u8 128^3 at 256x256 69, 56, 51, 51 (80); f32 (four registers a
+// voxel pair) 512^3 at 1024x1024 392, 342, 357, 352 (395).  The batched
+// kernel reads its frames from global memory and has no tail: there more
+// warps win (f32, 32 frames: 3.84 ms at K = 2 with 8 blocks, 4.57 with 5,
+// 4.33 at K = 4 with 5).
+#ifndef IVR_K_INT
+#define IVR_K_INT 6
 #endif
-constexpr bool kPair = IVR_CFG_PAIR != 0;
-// The second sample of a PAIR iteration reuses the first's corner-packed
-// cell when both lie in it (for u8 and u16 volumes; IVR_CELL_REUSE=0 turns
-// it off).  Measured on GB300: learned_1024 (u16) +4%; for f32 (16-byte
-// elements, twice the registers per cell) the plain march lost 4% and the
-// skipping march nothing, and keeping the last cell across iterations as
-// well cost more in spills than it saved (sorted_brick_512 -8%).
-#ifndef IVR_CELL_REUSE
-#define IVR_CELL_REUSE 1
+#ifndef IVR_K_F32
+#define IVR_K_F32 4
 #endif
-template <int DT> __host__ __device__ constexpr bool cell_reuse() { return IVR_CELL_REUSE != 0 && DT != IVR_F32; }
-// Likewise its LUT entry when both samples index the same one (every dtype;
-// IVR_LUT_REUSE=0 turns it off): +1-2% on learned_1024 and the plain march.
-// A copy of the LUT in each block's shared memory instead of reads through
-// L1 was 2-4% slower.
-#ifndef IVR_LUT_REUSE
-#define IVR_LUT_REUSE 1
-#endif
-constexpr bool kLutReuse = IVR_LUT_REUSE != 0;
-// Resident blocks per SM each kernel is compiled for.  More warps hide more
-// gather latency; past 8 blocks (64 registers) the compiler spills a little,
-// and measured on GB300 the occupancy still wins: 9 blocks (56 registers)
-// for the single-frame march, 9 (56) for the batched kernel, which reads
-// its frames from global memory (835 -> 1017 Gsamples/s from 6 blocks).
 #ifndef IVR_CFG_BLOCKS_PER_SM
-#define IVR_CFG_BLOCKS_PER_SM 9
+#define IVR_CFG_BLOCKS_PER_SM 5
 #endif
-constexpr int kCfgBlocksPerSm = IVR_CFG_BLOCKS_PER_SM;
-// judged launches (learned skipping) hold the exact march's state as well
-#ifndef IVR_JUDGE_BLOCKS_PER_SM
-#define IVR_JUDGE_BLOCKS_PER_SM 8
+#ifndef IVR_K_BATCH
+#define IVR_K_BATCH 2
 #endif
-constexpr int kJudgeBlocksPerSm = IVR_JUDGE_BLOCKS_PER_SM;
 #ifndef IVR_BATCH_BLOCKS_PER_SM
-#define IVR_BATCH_BLOCKS_PER_SM 9
+#define IVR_BATCH_BLOCKS_PER_SM 8
 #endif
+template <int DT> __host__ __device__ constexpr int cfg_k() { return DT == IVR_F32 ? IVR_K_F32 : IVR_K_INT; }
+constexpr int kCfgBlocksPerSm = IVR_CFG_BLOCKS_PER_SM;
+constexpr int kBatchK = IVR_K_BATCH;
 constexpr int kBatchBlocksPerSm = IVR_BATCH_BLOCKS_PER_SM;
+constexpr int kPeakBlocksPerSm = 9;  // the sampler alone (sample_peak_kernel)
 
 template <int DT> struct VoxT;
 template <> struct VoxT<IVR_U8> { using T = uint8_t; using V4 = uchar4; };
@@ -302,11 +296,7 @@ __device__ __forceinline__ float sample_cfg(const DevBrick &b, float ux, float u
 }
 
 // One voxel cell of a corner-packed copy as loaded: the two elements (slab
-// k and k+1), each holding the cell's four voxels of that slab.  A ray
-// stepping half a voxel takes its next sample in the same cell about half
-// the time; the march keeps the last cell it loaded, with its element
-// offset as the key, and loads again only when the cell changes.  The
-// values are the same voxels, so every sample is bitwise unchanged.
+// k and k+1), each holding the cell's four voxels of that slab.
 template <int DT> struct QuadCell;
 template <> struct QuadCell<IVR_U8> { unsigned lo, hi; };
 template <> struct QuadCell<IVR_U16> { uint2 lo, hi; };
@@ -524,149 +514,263 @@ __device__ __forceinline__ int cfg_first_ge(float t0, float dt, float idt, float
 }
 
 
-// One brick of the CONFIG march: samples tin_k <= t_i < tout_k of the ray's
-// lattice, front-to-back into acc.  One loop iteration takes one lattice
-// index (two with PAIR) for every lane, so the lanes of a warp stay in step.
-// With a macrocell grid a lane checks the cell of its sample (by the same
-// index arithmetic the sampler uses) only when it passes the exit of the last
-// opaque cell it checked.  A transparent cube's samples are stepped over to
-// just past its exit (or to two samples before it, where rounding at a face
-// leaves the last one in doubt), and successive cubes are leapt within the
-// same iteration; each skipped sample lies in a transparent cell, so it would
-// have had zero opacity and left acc unchanged.  An opaque cell's samples are
-// taken up to one past its exit without further checks.  Every sample that is
-// taken is computed exactly as without skipping.
-template <int DT, bool SKIP, bool CENSUS, bool PAIR>
-__device__ void march_cfg(const FrameDesc &f, const DevBrick &b, const uint8_t *empty, float dx, float dy, float dz,
-                          float idx, float idy, float idz, float t0, float dt, float idt, float4 &acc, bool &done,
-                          unsigned long long &nexec, unsigned long long &nlat)
+// K consecutive samples of a ray from lattice index fi: every load is issued
+// before the first interpolation.  Samples past the ray's run are harmless:
+// cell_cfg clamps the cells.
+template <int DT, int K>
+__device__ __forceinline__ void sample_run(const DevBrick &b, const VoxLattice &L, float fi, float (&s)[K])
+{
+    CellPos c[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const float fk = fi + (float) k;  // (float) (i + k): i < 2^24
+        c[k] = cell_cfg(b, fmaf(fk, L.sx, L.bx), fmaf(fk, L.sy, L.by), fmaf(fk, L.sz, L.bz));
+    }
+    if (b.quad) {
+        // Every sample loads its own cell, also where two share one: a copy
+        // of the neighbour's voxels would wait for that load, and its branch
+        // holds up the loads behind it (u16 learned frame 523 -> 358 us, f32
+        // unchanged).
+        QuadCell<DT> q[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) q[k] = quad_load<DT>(b, quad_key(b, c[k]));
+#pragma unroll
+        for (int k = 0; k < K; k++) s[k] = quad_interp<DT>(q[k], c[k]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; k++) s[k] = fetch_cfg<DT>(b, c[k]);
+    }
+}
+
+// The LUT entries of K samples, all loads issued before the first is
+// composited, and the first n of them composited front to back into acc.
+// True when the ray ended (alpha reached term).
+template <int K>
+__device__ __forceinline__ bool composite_run(const FrameDesc &f, const float (&s)[K], int n, float opac, float term,
+                                              float4 &acc)
+{
+    float4 e[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) e[k] = lut_at(f, (int) (s[k] * f.lut_scale) - f.lut_off);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (k >= n) break;
+        const float wgt = (1.0f - acc.w) * (e[k].w * opac);
+        acc.x = fmaf(wgt, e[k].x, acc.x);
+        acc.y = fmaf(wgt, e[k].y, acc.y);
+        acc.z = fmaf(wgt, e[k].z, acc.z);
+        acc.w = acc.w + wgt;
+        if (acc.w >= term) return true;
+    }
+    return false;
+}
+
+// A ray in a brick's macrocell grid: looks up the cell of sample i.
+// Returns true where the cell is opaque, with `next` one past the last sample
+// (i at least) taken in it without another look; else false, with `next` the
+// sample to look at after the leap over the transparent cube around it.
+// isx, isy, isz: lattice steps per voxel (about 1 / L.s).
+__device__ __forceinline__ bool look_cell(const DevBrick &b, const uint8_t *empty, const VoxLattice &L, float isx,
+                                          float isy, float isz, int i, int &next)
+{
+    const float fi = (float) i;
+    const CellPos c = cell_cfg(b, fmaf(fi, L.sx, L.bx), fmaf(fi, L.sy, L.by), fmaf(fi, L.sz, L.bz));
+    // the sample's macrocell: its voxel cell (the sampler's own index
+    // arithmetic) over the macrocell edge (cells are never negative: the
+    // sampler clamps them)
+    const int cs = b.cshift, edge = 1 << cs;
+    const int cj = c.j >> cs, ci = c.i >> cs, ck = c.k >> cs;
+    // r >= 1: the cube of cells within r-1 of this one is transparent
+    const int r = empty[(ck * b.mcy + ci) * b.mcx + cj];
+    const int rr = max(r, 1);
+    // the voxel plane of the face through which the ray leaves that cube (or
+    // this one opaque cell), per axis, and the lattice index of the exit;
+    // approximate, the margins absorb its rounding
+    const float fx = (float) ((L.sx > 0.0f ? cj + rr : cj - rr + 1) * edge);
+    const float fy = (float) ((L.sy > 0.0f ? ci + rr : ci - rr + 1) * edge);
+    const float fz = (float) ((L.sz > 0.0f ? ck + rr : ck - rr + 1) * edge);
+    const float qx = L.sx != 0.0f ? (fx - L.bx) * isx : FLT_MAX;
+    const float qy = L.sy != 0.0f ? (fy - L.by) * isy : FLT_MAX;
+    const float qz = L.sz != 0.0f ? (fz - L.bz) * isz : FLT_MAX;
+    const float q = fminf(fmaxf(fminf(qx, fminf(qy, qz)), 0.0f), (float) kMaxLattice);
+    const int iexit = (int) q;  // last lattice index at or before the exit
+    if (r == 0) {
+        next = max(iexit, i) + 1;
+        return true;
+    }
+    // Leap.  Sample positions are monotone in the lattice index along each
+    // axis and sample i lies in the cube, so when the last one before the
+    // exit (iexit) is still short of every exit face, so is every sample up
+    // to it: all are in the transparent cube, and the march resumes just past
+    // the exit.  Otherwise (rounding at a face) it resumes two samples
+    // earlier, where the next look decides again.  Every leap moves forward.
+    const float fe = (float) iexit;
+    const float ex = fmaf(fe, L.sx, L.bx), ey = fmaf(fe, L.sy, L.by), ez = fmaf(fe, L.sz, L.bz);
+    const bool inside = (L.sx > 0.0f ? ex < fx : L.sx < 0.0f ? ex >= fx : true) &&
+                        (L.sy > 0.0f ? ey < fy : L.sy < 0.0f ? ey >= fy : true) &&
+                        (L.sz > 0.0f ? ez < fz : L.sz < 0.0f ? ez >= fz : true);
+    next = max(i, inside ? iexit : iexit - 2) + 1;  // iexit + 1 or iexit - 1
+    return false;
+}
+
+// One brick of the CONFIG march without skipping: samples tin_k <= t_i <
+// tout_k of the ray's lattice, front-to-back into acc, K per iteration.
+template <int DT, int K>
+__device__ __forceinline__ void march_plain(const FrameDesc &f, const DevBrick &b, float dx, float dy, float dz,
+                                            float idx, float idy, float idz, float t0, float dt, float idt,
+                                            float4 &acc, bool &done)
+{
+    float tin, tout;
+    if (!ray_box_cfg(b.dconst, f.origx, f.origy, f.origz, dx, dy, dz, idx, idy, idz, tin, tout)) return;
+    const int i1 = cfg_first_ge(t0, dt, idt, tout);
+    const VoxLattice L = vox_lattice(b, f.origx, f.origy, f.origz, dx, dy, dz, t0, dt);
+    for (int i = cfg_first_ge(t0, dt, idt, tin); i < i1; i += K) {
+        float s[K];
+        sample_run<DT, K>(b, L, (float) i, s);
+        if (composite_run<K>(f, s, i1 - i, f.alpha, f.term_alpha, acc)) {
+            done = true;
+            return;
+        }
+    }
+}
+
+// The census of one brick (a diagnostic launch): the march's samples one by
+// one, each counted and its macrocell marked.
+template <int DT, bool SKIP>
+__device__ void march_census(const FrameDesc &f, const DevBrick &b, const uint8_t *empty, float dx, float dy, float dz,
+                             float idx, float idy, float idz, float t0, float dt, float idt, float4 &acc, bool &done,
+                             unsigned long long &nexec, unsigned long long &nlat)
 {
     float tin, tout;
     if (!ray_box_cfg(b.dconst, f.origx, f.origy, f.origz, dx, dy, dz, idx, idy, idz, tin, tout)) return;
     const int i0 = cfg_first_ge(t0, dt, idt, tin);
     const int i1 = cfg_first_ge(t0, dt, idt, tout);
-    if (CENSUS) {
-        nlat += (unsigned long long) max(i1 - i0, 0);
-        if (done) return;
-    }
-    const float opac = f.alpha, term = f.term_alpha;
+    nlat += (unsigned long long) max(i1 - i0, 0);
+    if (done) return;
     const VoxLattice L = vox_lattice(b, f.origx, f.origy, f.origz, dx, dy, dz, t0, dt);
-    // lattice steps per voxel (about 1 / L.s), for the exits of transparent
-    // cubes
     const float isx = idx * idt * b.vwx, isy = idy * idt * b.vwy, isz = idz * idt * b.vwz;
-    int icheck = i0;  // next lattice index whose cell must be checked
-    for (int i = i0; i < i1; i++) {
-        float fi = (float) i;
-        CellPos c0 = cell_cfg(b, fmaf(fi, L.sx, L.bx), fmaf(fi, L.sy, L.by), fmaf(fi, L.sz, L.bz));
-        // A lane leaps over transparent cubes within one iteration, until
-        // its sample lies in an opaque cell (or the brick ends), so that it
-        // samples beside the lanes that did not leap.  Every leap moves i
-        // forward and an opaque check leaves the loop, so it ends.
-        if (SKIP && i >= icheck) for (;;) {
-            // the sample's macrocell: its voxel cell (the sampler's own index
-            // arithmetic) over the macrocell edge (cells are never negative:
-            // the sampler clamps them)
-            const int cs = b.cshift, edge = 1 << cs;
-            const int cj = c0.j >> cs, ci = c0.i >> cs, ck = c0.k >> cs;
-            // r >= 1: the cube of cells within r-1 of this one is transparent
-            const int r = empty[(ck * b.mcy + ci) * b.mcx + cj];
-            const int rr = max(r, 1);
-            // the voxel plane of the face through which the ray leaves that
-            // cube (or this one opaque cell), per axis, and the lattice index
-            // of the exit; approximate, the margins absorb its rounding
-            const float fx = (float) ((L.sx > 0.0f ? cj + rr : cj - rr + 1) * edge);
-            const float fy = (float) ((L.sy > 0.0f ? ci + rr : ci - rr + 1) * edge);
-            const float fz = (float) ((L.sz > 0.0f ? ck + rr : ck - rr + 1) * edge);
-            const float qx = L.sx != 0.0f ? (fx - L.bx) * isx : FLT_MAX;
-            const float qy = L.sy != 0.0f ? (fy - L.by) * isy : FLT_MAX;
-            const float qz = L.sz != 0.0f ? (fz - L.bz) * isz : FLT_MAX;
-            const float q = fminf(fmaxf(fminf(qx, fminf(qy, qz)), 0.0f), (float) kMaxLattice);
-            const int iexit = (int) q;  // last lattice index at or before the exit
-            if (r != 0) {
-                // Leap.  Sample positions are monotone in the lattice index
-                // along each axis and sample i lies in the cube, so when the
-                // last one before the exit (iexit) is still short of every
-                // exit face, so is every sample up to it: all are in the
-                // transparent cube, and the march resumes just past the
-                // exit.  Otherwise (rounding at a face) it resumes two
-                // samples earlier, where the next check looks again.
-                const float fe = (float) iexit;
-                const float ex = fmaf(fe, L.sx, L.bx), ey = fmaf(fe, L.sy, L.by), ez = fmaf(fe, L.sz, L.bz);
-                const bool inside = (L.sx > 0.0f ? ex < fx : L.sx < 0.0f ? ex >= fx : true) &&
-                                    (L.sy > 0.0f ? ey < fy : L.sy < 0.0f ? ey >= fy : true) &&
-                                    (L.sz > 0.0f ? ez < fz : L.sz < 0.0f ? ez >= fz : true);
-                i = max(i, inside ? iexit : iexit - 2) + 1;  // iexit + 1 or iexit - 1
-                if (i >= i1) break;
-                fi = (float) i;
-                c0 = cell_cfg(b, fmaf(fi, L.sx, L.bx), fmaf(fi, L.sy, L.by), fmaf(fi, L.sz, L.bz));
+    int held = i0;  // samples i..held-1 lie in an opaque cell already looked up
+    for (int i = i0; i < i1;) {
+        if (SKIP && i >= held) {
+            int next;
+            if (!look_cell(b, empty, L, isx, isy, isz, i, next)) {
+                i = next;
                 continue;
             }
-            icheck = iexit + 1;
-            break;
+            held = next;
         }
-        if (SKIP && i >= i1) break;
-        // PAIR: two samples per iteration, both samples' loads in flight
-        // before either is composited.  The second is only composited when
-        // it comes before the next cell check and the first did not end the
-        // ray; sample_cfg clamps its indices, so computing it is always safe.
-        if (PAIR && !CENSUS) {
-            const int lim = SKIP ? min(i1, icheck) : i1;
-            const float f1 = fi + 1.0f;  // (float) (i + 1): i < 2^24
-            float s0, s1;
-            if (cell_reuse<DT>() && b.quad) {
-                const CellPos c1 = cell_cfg(b, fmaf(f1, L.sx, L.bx), fmaf(f1, L.sy, L.by), fmaf(f1, L.sz, L.bz));
-                const unsigned k0 = quad_key(b, c0), k1 = quad_key(b, c1);
-                const QuadCell<DT> q0 = quad_load<DT>(b, k0);
-                QuadCell<DT> q1 = q0;
-                if (k1 != k0) q1 = quad_load<DT>(b, k1);
-                s0 = quad_interp<DT>(q0, c0);
-                s1 = quad_interp<DT>(q1, c1);
-            } else {
-                s0 = fetch_cfg<DT>(b, c0);
-                s1 = sample_cfg<DT>(b, fmaf(f1, L.sx, L.bx), fmaf(f1, L.sy, L.by), fmaf(f1, L.sz, L.bz));
-            }
-            const int x0 = (int) (s0 * f.lut_scale) - f.lut_off, x1 = (int) (s1 * f.lut_scale) - f.lut_off;
-            const float4 e0 = lut_at(f, x0);
-            float4 e1 = e0;
-            if (!kLutReuse || x1 != x0) e1 = lut_at(f, x1);  // the same entry: no second load
-            float wgt = (1.0f - acc.w) * (e0.w * opac);
-            acc.x = fmaf(wgt, e0.x, acc.x);
-            acc.y = fmaf(wgt, e0.y, acc.y);
-            acc.z = fmaf(wgt, e0.z, acc.z);
-            acc.w = acc.w + wgt;
-            if (acc.w >= term) {
-                done = true;
-                return;
-            }
-            if (i + 1 < lim) {
-                wgt = (1.0f - acc.w) * (e1.w * opac);
-                acc.x = fmaf(wgt, e1.x, acc.x);
-                acc.y = fmaf(wgt, e1.y, acc.y);
-                acc.z = fmaf(wgt, e1.z, acc.z);
-                acc.w = acc.w + wgt;
-                if (acc.w >= term) {
-                    done = true;
-                    return;
-                }
-                i++;
-            }
-            continue;
-        }
-        const float s = fetch_cfg<DT>(b, c0);
-        if (CENSUS) {
-            nexec++;
-            b.touched[((long long) (c0.k >> b.cshift) * b.mcy + (c0.i >> b.cshift)) * b.mcx + (c0.j >> b.cshift)] = 1;
-        }
-        const float4 e = lut_at(f, (int) (s * f.lut_scale) - f.lut_off);
-        const float al = e.w * opac;
-        const float wgt = (1.0f - acc.w) * al;
-        acc.x = fmaf(wgt, e.x, acc.x);
-        acc.y = fmaf(wgt, e.y, acc.y);
-        acc.z = fmaf(wgt, e.z, acc.z);
-        acc.w = acc.w + wgt;
-        if (acc.w >= term) {
+        const float fi = (float) i;
+        const CellPos c = cell_cfg(b, fmaf(fi, L.sx, L.bx), fmaf(fi, L.sy, L.by), fmaf(fi, L.sz, L.bz));
+        nexec++;
+        b.touched[((long long) (c.k >> b.cshift) * b.mcy + (c.i >> b.cshift)) * b.mcx + (c.j >> b.cshift)] = 1;
+        const float s[1] = {fetch_cfg<DT>(b, c)};
+        if (composite_run<1>(f, s, 1, f.alpha, f.term_alpha, acc)) {
             done = true;
             return;
+        }
+        i++;
+    }
+}
+
+// Samples a lane looks ahead for (at most 255: a run's length has 8 bits),
+// and runs it can hold.  Learned 1024^3 / f32 512^3 frames, us: 549 / 373 at
+// 32 samples, 527 / 361 at 64, 518 / 356 at 128.
+constexpr int kRunSamples = 128;
+constexpr int kRunMax = 8;
+constexpr unsigned kFullWarp = 0xffffffffu;
+static_assert(kRunSamples < 256, "run lengths have 8 bits");
+
+// One brick of the CONFIG march with a skipping grid, in two alternating
+// steps.  (1) Each lane walks its ray over the macrocell grid and notes the
+// runs of lattice indices that lie in opaque cells, until it has
+// kRunSamples of them: transparent cubes are leapt over, runs of
+// neighbouring opaque cells join.  (2) All lanes sample and composite their
+// runs.  A warp whose lanes checked a cell wherever one of them left its
+// last one ran that check (a dependent load and some 60 instructions) in
+// nearly every iteration; here the lanes walk together and sample together,
+// each with the same number of samples at hand.  The samples taken are the
+// same as when every cell is checked as it is reached, and every sample is
+// computed exactly as without skipping.  `runs` is the lane's column of a
+// [kRunMax][kThreads] shared array: start in the low 24 bits, length above.
+// Every lane of the warp calls this (`in` false: without a ray), and the
+// loops are the warp's, so that lanes which leave a step early wait for the
+// others instead of taking the next step on their own (that took twice the
+// time).  Bound by the latency of the longest rays: of a 354 us f32 frame
+// (512^3, 1024x1024) the SMs have work for about 70%, with 43% of all issue
+// slots used.
+template <int DT, int K>
+__device__ __forceinline__ void march_runs(const FrameDesc &f, const DevBrick &b, const uint8_t *empty,
+                                           unsigned *runs, bool in, float dx, float dy, float dz, float idx,
+                                           float idy, float idz, float t0, float dt, float idt, float4 &acc,
+                                           bool &done)
+{
+    float tin, tout;
+    in = in && ray_box_cfg(b.dconst, f.origx, f.origy, f.origz, dx, dy, dz, idx, idy, idz, tin, tout);
+    int i = in ? cfg_first_ge(t0, dt, idt, tin) : 0;  // the next lattice index to look at
+    int i1 = in ? cfg_first_ge(t0, dt, idt, tout) : 0;
+    const float opac = f.alpha, term = f.term_alpha;
+    const VoxLattice L = vox_lattice(b, f.origx, f.origy, f.origz, dx, dy, dz, t0, dt);
+    const float isx = idx * idt * b.vwx, isy = idy * idt * b.vwy, isz = idz * idt * b.vwz;
+    int held = i;  // indices i..held-1 lie in an opaque cell already checked
+    while (__any_sync(kFullWarp, i < i1)) {
+        int nr = 0, n = 0;       // runs noted, samples in them
+        int start = 0, len = 0;  // the run being built
+        bool walk = i < i1;
+        while (__any_sync(kFullWarp, walk)) {
+            if (!walk) continue;
+            if (i >= held) {
+                int next;
+                if (look_cell(b, empty, L, isx, isy, isz, i, next)) held = next;
+                else i = next;
+            }
+            if (i < held && i < i1) {
+                const bool gap = len > 0 && start + len != i;
+                if (gap && nr == kRunMax - 1) {
+                    walk = false;  // no room for another run
+                } else {
+                    if (gap) {
+                        runs[nr * kThreads] = (unsigned) start | (unsigned) len << 24;
+                        nr++;
+                        len = 0;
+                    }
+                    if (len == 0) start = i;
+                    const int take = min(min(held, i1) - i, kRunSamples - n);
+                    len += take;
+                    n += take;
+                    i += take;
+                }
+            }
+            walk = walk && i < i1 && n < kRunSamples;
+        }
+        if (len > 0) {
+            runs[nr * kThreads] = (unsigned) start | (unsigned) len << 24;
+            nr++;
+        }
+        // the runs' samples, K at a time, their loads in flight before the
+        // first is composited; those past a run's end are not composited
+        // (cell_cfg clamps the cells, so computing them is always safe)
+        len = 0;
+        for (int r = 0;;) {
+            if (len == 0 && r < nr) {
+                const unsigned w = runs[r * kThreads];
+                start = (int) (w & 0xffffffu);
+                len = (int) (w >> 24);
+                r++;
+            }
+            if (!__any_sync(kFullWarp, len > 0)) break;
+            if (len == 0) continue;
+            float s[K];
+            sample_run<DT, K>(b, L, (float) start, s);
+            if (composite_run<K>(f, s, len, opac, term, acc)) {
+                done = true;
+                nr = 0;
+                len = 0;
+                i = i1;
+            } else {
+                const int take = min(len, K);
+                start += take;
+                len -= take;
+            }
         }
     }
 }
@@ -733,16 +837,18 @@ __global__ void __launch_bounds__(kThreads) march_ref_kernel(const __grid_consta
     count_exec(f, nexec);
 }
 
-// One CONFIG ray: pixel (i, j) of the viewport, all bricks front to back,
-// skipping by the bricks' grids, or by the exact grids f.exact when exact.
-template <int DT, bool SKIP, bool CENSUS, bool PAIR>
-__device__ __forceinline__ float4 ray_cfg(const FrameDesc &f, int i, int j, unsigned long long &nexec,
-                                          unsigned long long &nlat, bool exact = false)
+// One CONFIG ray per lane: pixel (i, j) of the viewport, all bricks front to
+// back, skipping by the bricks' grids, or by the exact grids f.exact when
+// exact.  Every lane of the warp calls it; one with `live` false has no ray.
+template <int DT, bool SKIP, bool CENSUS, int K>
+__device__ __forceinline__ float4 ray_cfg(const FrameDesc &f, int i, int j, bool live, unsigned long long &nexec,
+                                          unsigned long long &nlat, unsigned *runs, bool exact = false)
 {
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     bool any = false;
     for (int k = 0; k < f.nb; k++) any |= in_rect(f.b[k], i, j);
-    if (!any) return acc;
+    live = live && any;
+    if (!__any_sync(kFullWarp, live)) return acc;
     // ctm * (u, v, 5) at the pixel centre
     const float u = f.left + ((float) j + 0.5f) * f.du;
     const float v = f.bottom + ((float) i + 0.5f) * f.dv;
@@ -751,37 +857,42 @@ __device__ __forceinline__ float4 ray_cfg(const FrameDesc &f, int i, int j, unsi
     const float dz = f.ctm[6] * u + f.ctm[7] * v + f.ctm[8] * f.eyen;
     const float idx = 1.0f / dx, idy = 1.0f / dy, idz = 1.0f / dz;
     float tin, tout;
-    if (!ray_box_cfg(f.gdconst, f.origx, f.origy, f.origz, dx, dy, dz, idx, idy, idz, tin, tout)) return acc;
-    const float t0 = tin > 0.0f ? tin : 0.0f;
+    live = live && ray_box_cfg(f.gdconst, f.origx, f.origy, f.origz, dx, dy, dz, idx, idy, idz, tin, tout);
+    const float t0 = live && tin > 0.0f ? tin : 0.0f;
     const float len = sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
     const float dt = f.step / len;
-    bool done = !(dt > 0.0f);
+    bool done = !live || !(dt > 0.0f);
     const float idt = 1.0f / dt;
-    for (int s = 0; s < f.nb && (CENSUS || !done); s++) {
+    for (int s = 0; s < f.nb; s++) {
         const int k = f.order[s];
         if (f.single >= 0 && k != f.single) continue;
         const DevBrick &b = f.b[k];
-        if (!in_rect(b, i, j)) continue;
+        const bool in = (CENSUS ? live : !done) && in_rect(b, i, j);
+        if (!__any_sync(kFullWarp, in)) continue;
         const uint8_t *empty = exact ? f.exact[k] : b.empty;
-        if (SKIP && empty != nullptr)
-            march_cfg<DT, true, CENSUS, PAIR>(f, b, empty, dx, dy, dz, idx, idy, idz, t0, dt, idt, acc, done, nexec,
-                                              nlat);
-        else
-            march_cfg<DT, false, CENSUS, PAIR>(f, b, empty, dx, dy, dz, idx, idy, idz, t0, dt, idt, acc, done, nexec,
-                                               nlat);
+        if constexpr (CENSUS) {
+            if (in && SKIP && empty != nullptr)
+                march_census<DT, true>(f, b, empty, dx, dy, dz, idx, idy, idz, t0, dt, idt, acc, done, nexec, nlat);
+            else if (in)
+                march_census<DT, false>(f, b, empty, dx, dy, dz, idx, idy, idz, t0, dt, idt, acc, done, nexec, nlat);
+        } else if (SKIP && empty != nullptr) {
+            march_runs<DT, K>(f, b, empty, runs, in, dx, dy, dz, idx, idy, idz, t0, dt, idt, acc, done);
+        } else if (in) {
+            march_plain<DT, K>(f, b, dx, dy, dz, idx, idy, idz, t0, dt, idt, acc, done);
+        }
     }
     return acc;
 }
 
 // One pixel of the output window (ow, oh) = (oj, oi).
-template <int DT, bool SKIP, bool CENSUS, bool PAIR>
+template <int DT, bool SKIP, bool CENSUS, int K>
 __device__ __forceinline__ float4 pixel_cfg(const FrameDesc &f, int oi, int oj, float4 *out32, uchar4 *out8,
-                                            unsigned long long &nexec, unsigned long long &nlat, bool exact = false)
+                                            unsigned long long &nexec, unsigned long long &nlat, unsigned *runs)
 {
-    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (oj >= f.out_w || oi >= f.out_h) return acc;
+    const bool in_window = oj < f.out_w && oi < f.out_h;
     const int j = f.out_x + oj, i = f.out_y + oi;
-    if (i < f.vh && j < f.vw) acc = ray_cfg<DT, SKIP, CENSUS, PAIR>(f, i, j, nexec, nlat, exact);
+    const float4 acc = ray_cfg<DT, SKIP, CENSUS, K>(f, i, j, in_window && i < f.vh && j < f.vw, nexec, nlat, runs);
+    if (!in_window) return acc;
     const long long o = (long long) oi * f.out_w + oj;
     if (out32) out32[o] = acc;
     if (out8) out8[o] = make_uchar4(q8(acc.x), q8(acc.y), q8(acc.z), q8(acc.w));
@@ -1002,12 +1113,23 @@ __host__ __device__ inline long long judged_tiles(long long ntiles, int stride, 
     return ntiles > phase ? (ntiles - phase + stride - 1) / stride : 0;
 }
 
-// CONFIG kernel, persistent: every warp takes 8x4 pixel tiles from the
-// view's ticket counter until none are left, so warps that drew short rays
-// pick up more work instead of idling while the grid's last blocks finish.
-// With f.perm the n-th ticket renders tile perm[n] (costliest first).
-// A gated launch (f.gate set) renders only if *f.gate != 0; otherwise its
-// warps take their share of tickets (tiles + one failed take each) and leave.
+// Tickets a launch of `total` tiles on `nwarps` warps takes: each tile after
+// the warps' first ones, and one failed take per warp; none when the warps'
+// first tiles are all.
+__host__ __device__ inline long long launch_tickets(long long total, long long nwarps)
+{
+    return total > nwarps ? total : 0;
+}
+
+// CONFIG kernel, persistent: every warp takes one 8x4 pixel tile by its rank
+// and then tiles from the view's ticket counter until none are left, so warps
+// that drew short rays pick up more work instead of idling while the grid's
+// last blocks finish.  Taken from the counter too, the first (costliest)
+// tiles went four to a block to the SMs that started first: a 256x256 frame
+// took 86 us, with the busiest SM at 55% and the mean at 7%, and takes 75 by
+// rank.  With f.perm the n-th tile is perm[n] (costliest first).
+// A gated launch (f.gate set) renders only if *f.gate != 0; otherwise it
+// takes its share of tickets (launch_tickets) and leaves.
 // JUDGE (learned skipping): the first tickets re-march the judged tiles
 // (judge_phase modulo judge_stride) with the exact grids into f.judge8,
 // each on its own warp, so that a judged heavy tile does not double the
@@ -1016,27 +1138,36 @@ __host__ __device__ inline long long judged_tiles(long long ntiles, int stride, 
 // exact grids and nothing is re-marched.  judge_compare_kernel gives the
 // verdict afterwards.
 template <int DT, bool SKIP, bool CENSUS, bool JUDGE>
-__global__ void __launch_bounds__(kThreads, JUDGE ? kJudgeBlocksPerSm : kCfgBlocksPerSm)
+__global__ void __launch_bounds__(kThreads, kCfgBlocksPerSm)
     march_cfg_kernel(const __grid_constant__ FrameDesc f, float4 *out32, uchar4 *out8)
 {
+    __shared__ unsigned s_runs[SKIP && !CENSUS ? kRunMax * kThreads : 1];
     unsigned long long nexec = 0, nlat = 0;
     const int lane = threadIdx.x & 31;
     const int tiles_x = (f.out_w + 7) >> 3;
     const long long ntiles = (long long) tiles_x * ((f.out_h + 3) >> 2);
+    const long long njudged = JUDGE ? judged_tiles(ntiles, f.judge_stride, f.judge_phase) : 0;
+    const long long total = ntiles + njudged, nwarps = (long long) gridDim.x * (kThreads / 32);
     if (f.gate != nullptr && *f.gate == 0) {
-        // no fallback: the launch's share of tickets (every tile, and one
-        // failed take per warp) in one add instead of one per warp
-        if (blockIdx.x == 0 && threadIdx.x == 0)
-            atomicAdd(f.tickets, (unsigned long long) ntiles + (unsigned long long) gridDim.x * (blockDim.x >> 5));
+        // no fallback: the launch's share of tickets in one add
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(f.tickets, (unsigned long long) launch_tickets(total, nwarps));
         return;
     }
     const bool exact = JUDGE && *(volatile const int *) f.learned_bad != 0;
-    const long long njudged = JUDGE ? judged_tiles(ntiles, f.judge_stride, f.judge_phase) : 0;
-    for (;;) {
-        unsigned long long ticket = 0;
-        if (lane == 0) ticket = atomicAdd(f.tickets, 1ull);
-        const long long q = (long long) (__shfl_sync(0xffffffffu, ticket, 0) - f.ticket_base);
-        if (q >= ntiles + njudged) break;
+    // the warp's first tile is its rank among the launch's warps, counted
+    // across the blocks: the costliest tiles spread over the SMs, one each
+    // before any has two
+    long long q = (long long) (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    for (bool first = true;; first = false) {
+        if (!first) {
+            if (total <= nwarps) break;
+            unsigned long long ticket = 0;
+            if (lane == 0) ticket = atomicAdd(f.tickets, 1ull);
+            q = nwarps + (long long) (__shfl_sync(0xffffffffu, ticket, 0) - f.ticket_base);
+            if (q >= total) break;
+        } else if (q >= total) {
+            continue;
+        }
         // a judged tile (re-marched with the exact grids into judge8) or a
         // render tile, through one copy of the march
         const bool judge = JUDGE && q < njudged;
@@ -1054,8 +1185,9 @@ __global__ void __launch_bounds__(kThreads, JUDGE ? kJudgeBlocksPerSm : kCfgBloc
         const int oi = (int) (tile / tiles_x) * 4 + (lane >> 3), oj = (int) (tile % tiles_x) * 8 + (lane & 7);
         const bool in_window = oi < f.out_h && oj < f.out_w;
         const int i = f.out_y + oi, j = f.out_x + oj;
-        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (in_window && i < f.vh && j < f.vw) acc = ray_cfg<DT, SKIP, CENSUS, kPair>(f, i, j, nexec, nlat, judge || exact);
+        const float4 acc =
+            ray_cfg<DT, SKIP, CENSUS, cfg_k<DT>()>(
+                f, i, j, in_window && i < f.vh && j < f.vw, nexec, nlat, s_runs + threadIdx.x, judge || exact);
         const uchar4 a8 = make_uchar4(q8(acc.x), q8(acc.y), q8(acc.z), q8(acc.w));
         if (judge) {
             f.judge8[q * 32 + lane] = a8;
@@ -1133,7 +1265,7 @@ __device__ __forceinline__ float sample_layout(const DevBrick &b, const SamplerT
 }
 
 template <int DT, int LAYOUT>
-__global__ void __launch_bounds__(kThreads, kCfgBlocksPerSm) sample_peak_kernel(const __grid_constant__ FrameDesc f,
+__global__ void __launch_bounds__(kThreads, kPeakBlocksPerSm) sample_peak_kernel(const __grid_constant__ FrameDesc f,
                                                                                 SamplerTex tex, int steps,
                                                                                 float4 *out)
 {
@@ -1153,21 +1285,8 @@ __global__ void __launch_bounds__(kThreads, kCfgBlocksPerSm) sample_peak_kernel(
     const float loy = 1.0f, hiy = sy - 1.0f;
     const float loz = 1.0f, hiz = sz - 1.0f;
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    QuadCell<DT> qlast{};
-    unsigned qkey = 0;
     for (int i = 0; i < steps; i++) {
-        float s;
-        if (LAYOUT == IVR_SAMPLER_QUADS && cell_reuse<DT>()) {
-            // the march's sampler: samples taken in pairs, the second
-            // reusing the first's cell when both lie in it
-            const CellPos c = cell_cfg(b, x, y, z);
-            const unsigned k = quad_key(b, c);
-            if (!(i & 1) || k != qkey) qlast = quad_load<DT>(b, k);
-            qkey = k;
-            s = quad_interp<DT>(qlast, c);
-        } else {
-            s = sample_layout<DT, LAYOUT>(b, tex, x, y, z);
-        }
+        const float s = sample_layout<DT, LAYOUT>(b, tex, x, y, z);
         const float4 e = lut_at(f, (int) (s * f.lut_scale) - f.lut_off);
         const float wgt = (1.0f - acc.w) * (e.w * f.alpha);
         acc.x = fmaf(wgt, e.x, acc.x);
@@ -1236,13 +1355,11 @@ cudaError_t launch_dt(const FrameDesc &f, float4 *o32, uchar4 *o8, cudaStream_t 
                     : judge  ? march_cfg_kernel<DT, true, false, true>
                     : skip   ? march_cfg_kernel<DT, true, false, false>
                              : march_cfg_kernel<DT, false, false, false>;
-        const int blocks = persistent_grid(kern, 0);
-        // every tile (and, judged, every re-march) is taken once and every
-        // warp ends on one failed take
         const long long ntiles = (long long) ((f.out_w + 7) >> 3) * ((f.out_h + 3) >> 2);
-        if (warps_launched)
-            *warps_launched = ntiles + (judge ? judged_tiles(ntiles, f.judge_stride, f.judge_phase) : 0) +
-                              (long long) blocks * (kThreads / 32);
+        const long long total = ntiles + (judge ? judged_tiles(ntiles, f.judge_stride, f.judge_phase) : 0);
+        constexpr int kWarps = kThreads / 32;
+        const int blocks = (int) std::min((long long) persistent_grid(kern, 0), (total + kWarps - 1) / kWarps);
+        if (warps_launched) *warps_launched = launch_tickets(total, (long long) blocks * kWarps);
         kern<<<blocks, kThreads, 0, s>>>(f, o32, o8);
         return cudaGetLastError();
     }
@@ -1270,6 +1387,7 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocksPerSm)
                        unsigned long long *ticket)
 {
     constexpr int TH = 32 / TW;
+    __shared__ unsigned s_runs[kRunMax * kThreads];
     const int lane = threadIdx.x & 31;
     const int n = hdr->nitems;
     const long long total = hdr->total_tiles;
@@ -1287,8 +1405,9 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocksPerSm)
         }
         const BatchItem &it = items[lo];
         const long long tile = g - it.tile0;
-        pixel_cfg<DT, true, false, PAIR>(it.f, (int) (tile / it.tiles_x) * TH + lane / TW,
-                                        (int) (tile % it.tiles_x) * TW + lane % TW, it.out32, it.out8, nexec, nlat);
+        pixel_cfg<DT, true, false, PAIR ? kBatchK : 1>(it.f, (int) (tile / it.tiles_x) * TH + lane / TW,
+                                        (int) (tile % it.tiles_x) * TW + lane % TW, it.out32, it.out8, nexec, nlat,
+                                        s_runs + threadIdx.x);
     }
 }
 
