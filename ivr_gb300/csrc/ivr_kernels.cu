@@ -255,22 +255,30 @@ __global__ void __launch_bounds__(1024) hist_kernel(const T *__restrict__ data, 
     }
 }
 
-// More bins than four ranges hold (float volumes of a wide range): counters
-// in global memory, runs added at once.
-__global__ void hist_global_kernel(const float *__restrict__ data, long long n, MinArg mn, int hsize, int *hist)
+// The same with the counters in global memory: for more bins than two ranges
+// hold (float volumes of a wide range), and for volumes too small to pay for
+// clearing and adding up shared counters.
+template <typename T>
+__global__ void hist_global_kernel(const T *__restrict__ data, long long n, MinArg mn, int hsize, int *hist)
 {
     const float fmin = mn.dev ? __ldg(mn.dev) : mn.v;
-    int cur = -1, run = 0;
+    int zero = 0, cur = -1, run = 0;
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
-        const int b = (int) (__ldg(data + i) - fmin);
-        if (b != cur) {
-            if ((unsigned) cur < (unsigned) hsize) atomicAdd(&hist[cur], run);
-            cur = b;
-            run = 0;
+        const int b = (int) ((float) __ldg(data + i) - fmin);
+        if (b == 0) {
+            zero++;
+        } else {
+            if (b != cur) {
+                if ((unsigned) cur < (unsigned) hsize) atomicAdd(&hist[cur], run);
+                cur = b;
+                run = 0;
+            }
+            run++;
         }
-        run++;
     }
     if ((unsigned) cur < (unsigned) hsize) atomicAdd(&hist[cur], run);
+    zero = __reduce_add_sync(0xffffffffu, zero);
+    if ((threadIdx.x & 31) == 0 && zero) atomicAdd(&hist[0], zero);
 }
 
 // Macrocell min/max: with edge `cell`, cell (cx,cy,cz) spans voxels
@@ -482,7 +490,14 @@ __global__ void minmax_final_kernel(const float *partial, int nparts, float *min
 constexpr int kHistBlocks = kSms;           // one block an SM
 constexpr int kHistSmem = 224 * 1024;       // shared memory a block may ask for
 constexpr int kHistBins = kHistSmem / 4;    // counters in it
-constexpr int kHistRanges = 4;              // ranges before the bins move to global memory
+constexpr int kHistRanges = 2;              // ranges before the counters move to global memory:
+                                            // at four (229,375 bins, 256^3 f32 voxels) a call
+                                            // took 130 us against 88 in global memory, at two
+                                            // (65,536 bins, 256^3 u16) 75 against 87
+constexpr int kHistSmall = 128;             // voxels per bin below which global counters win:
+                                            // 256 bins, u8: 32^3 (128 a bin) 25.5 us shared, 24.4
+                                            // global, 48^3 (432) 25.7 and 33.0; 65,536 bins, u16:
+                                            // 160^3 (62) 52 and 47, 256^3 (256) 75 and 87
 
 template <typename T>
 cudaError_t hist_launch(const T *data, long long n, MinArg mn, int hsize, int *hist, cudaStream_t s)
@@ -504,20 +519,23 @@ cudaError_t hist_launch(const T *data, long long n, MinArg mn, int hsize, int *h
     return cudaGetLastError();
 }
 
+template <typename T>
+cudaError_t hist_dt(const T *data, long long n, MinArg mn, int hsize, int *hist, cudaStream_t s)
+{
+    if (sizeof(T) < 4) hsize = std::min(hsize, 65536);  // integer voxels: the bins above stay empty
+    if (hsize > kHistRanges * kHistBins || n < (long long) kHistSmall * hsize) {
+        hist_global_kernel<<<grid_for(n, 256), 256, 0, s>>>(data, n, mn, hsize, hist);
+        return cudaGetLastError();
+    }
+    return hist_launch(data, n, mn, hsize, hist, s);
+}
+
 cudaError_t hist_any(const void *data, int dtype, long long n, MinArg mn, int hsize, int *hist, cudaStream_t s)
 {
-    if ((long long) hsize > (long long) kHistRanges * kHistBins) {
-        // integer voxels have at most 65,536 values: bins above are empty
-        if (dtype == IVR_F32) {
-            hist_global_kernel<<<grid_for(n, 256), 256, 0, s>>>((const float *) data, n, mn, hsize, hist);
-            return cudaGetLastError();
-        }
-        hsize = 65536;
-    }
     switch (dtype) {
-    case IVR_U8: return hist_launch((const uint8_t *) data, n, mn, hsize, hist, s);
-    case IVR_U16: return hist_launch((const uint16_t *) data, n, mn, hsize, hist, s);
-    default: return hist_launch((const float *) data, n, mn, hsize, hist, s);
+    case IVR_U8: return hist_dt((const uint8_t *) data, n, mn, hsize, hist, s);
+    case IVR_U16: return hist_dt((const uint16_t *) data, n, mn, hsize, hist, s);
+    default: return hist_dt((const float *) data, n, mn, hsize, hist, s);
     }
 }
 

@@ -18,15 +18,16 @@ def volume(dtype, shape, top, seed=1):
 
 
 # shapes whose voxel count leaves every remainder of a 16-byte load, one
-# smaller than a load, and one with more than one trip per thread; value
-# ranges below and above 32 copies, one range, two ranges, and (f32) more
-# bins than the shared-memory ranges hold
+# smaller than a load, and one with more than one trip per thread; voxels per
+# bin on both sides of the shared counters' rule (128); and for the shared
+# ones 32, 2 and 1 copies, one range, two ranges, and more bins than two hold
 @pytest.mark.parametrize("dtype,shape,top", [
-    ("u8", (2, 2, 2), 255), ("u8", (5, 7, 11), 255), ("u8", (160, 170, 181), 255), ("u8", (16, 16, 16), 3),
-    ("u16", (3, 3, 5), 65535), ("u16", (31, 33, 35), 896), ("u16", (64, 65, 67), 28671), ("u16", (64, 64, 66), 57344),
-    ("u16", (130, 129, 127), 65535), ("f32", (3, 3, 3), 255.0), ("f32", (97, 101, 103), 255.0),
-    ("f32", (33, 34, 35), 57343.0), ("f32", (40, 40, 41), 57344.5), ("f32", (40, 41, 42), 229375.0),
-    ("f32", (40, 41, 43), 229376.5), ("f32", (48, 40, 44), 1.0e6)])
+    ("u8", (2, 2, 2), 255), ("u8", (5, 7, 11), 255), ("u8", (16, 16, 16), 3), ("u8", (32, 32, 31), 255),
+    ("u8", (32, 32, 32), 255), ("u8", (160, 170, 181), 255), ("u16", (3, 3, 5), 65535), ("u16", (63, 64, 65), 896),
+    ("u16", (31, 33, 35), 28671), ("u16", (130, 130, 113), 14335), ("u16", (205, 205, 204), 65535),
+    ("f32", (3, 3, 3), 255.0), ("f32", (97, 101, 103), 255.0), ("f32", (40, 40, 40), 57343.0),
+    ("f32", (196, 195, 194), 57343.0), ("f32", (245, 245, 246), 114687.0), ("f32", (245, 246, 247), 114688.0),
+    ("f32", (48, 40, 44), 1.0e6)])
 def test_minmax_and_histogram_match_the_oracle(ctx, oracle_mod, dtype, shape, top):
     vol = volume(dtype, shape, top)
     omn, omx, ohist = oracle_mod.minmax_histogram(vol)
