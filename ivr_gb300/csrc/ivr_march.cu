@@ -180,6 +180,181 @@ __device__ __forceinline__ float sample_ref(const DevBrick &b, float x, float y,
     return c0 * (1.0f - zd) + c1 * zd;
 }
 
+// Two floats in one 64-bit register pair: sm_100's packed FP32 instructions
+// do both operations in one issue slot.  The assembler contracts a packed
+// product that only feeds a packed sum into one fma, whatever the rounding
+// qualifiers and flags say (measured: 246,536 of 2^20 sums differ), so F2 has
+// no product-then-sum: such steps stay scalar, where it does not.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ void f2_split(F2 x, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
+// x / c for a divisor fixed over a ray: h = 1/c rounded to nearest, l the
+// rest of 1/c.  fmaf(x, h, x * l) is within one rounding of a relative 2^-46
+// of the quotient, so it is one of its two float neighbours; the remainder of
+// that is then exact in one fmaf, and adding it times h gives the quotient
+// rounded to nearest (Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", 1990, theorem on the final division step;
+// the two-word reciprocal is Brisebarre and Muller's, "Correctly rounded
+// multiplication by arbitrary precision constants", 2008).  Neither bound
+// holds near the ends of the exponent range: callers pass 0 < |x| in
+// [kDivMin, kDivMax] or x = 0, and divisors in the same range.
+constexpr float kDivMin = 8.673617379884035e-19f, kDivMax = 1.152921504606847e18f;  // 2^-60, 2^60
+struct FixedDiv {
+    F2 mc, h, l;  // -c, 1/c, the rest of 1/c, for both lanes
+    __device__ __forceinline__ explicit FixedDiv(float d)
+    {
+        const float r = 1.0f / d;
+        mc = f2(-d);
+        h = f2(r);
+        l = f2(fmaf(-d, r, 1.0f) * r);
+    }
+    __device__ __forceinline__ F2 operator()(F2 x) const
+    {
+        const F2 q = f2_fma(x, h, x * l);
+        return f2_fma(f2_fma(q, mc, x), h, q);
+    }
+};
+
+// Whether every division that sample_ref makes along the ray is one that
+// FixedDiv rounds as IEEE division does.  The positions x = o + d t are
+// compared with a brick edge and cell corners; where those, or o, are at
+// least 2^-30, the difference of two floats near each other is a multiple of
+// the smaller one's last place, so it is 0 or at least 2^-57.  An edge at 0
+// (inner bricks) seen from o = 0 needs d t away from 0 as well.
+__device__ __forceinline__ bool ref_fast_axis(float o, float d, float bmin, float extent, float tin)
+{
+    const float tiny = 9.313225746154785e-10f, huge = 1.099511627776e12f;  // 2^-30, 2^40
+    if (!(fabsf(o) <= huge && fabsf(d) <= huge && extent >= tiny && extent <= huge && fabsf(bmin) <= huge)) return false;
+    if (fabsf(bmin) >= tiny) return true;
+    if (bmin != 0.0f) return false;
+    if (fabsf(o) >= tiny) return true;
+    return o == 0.0f && (d == 0.0f || (fabsf(d) >= tiny && tin >= 1.0e-6f));
+}
+__device__ __forceinline__ bool ref_fast(const FrameDesc &f, const DevBrick &b, float dx, float dy, float dz, float tin)
+{
+    return fabsf(tin) <= 65536.0f && ref_fast_axis(f.origx, dx, b.bminx, b.w, tin) &&
+           ref_fast_axis(f.origy, dy, b.bminy, b.h, tin) && ref_fast_axis(f.origz, dz, b.bminz, b.d, tin);
+}
+
+// A ray's REF sampler in one brick: sample_ref with its nine divisions, all
+// by the brick's extents or dims, as FixedDivs, and (u8, u16) the eight
+// voxels from the corner-packed copy in two loads.
+struct RefSampler {
+    FixedDiv w, h, d, nx, ny, nz;
+    __device__ __forceinline__ explicit RefSampler(const DevBrick &b)
+        : w(b.w), h(b.h), d(b.d), nx((float) b.nx), ny((float) b.ny), nz((float) b.nz)
+    {
+    }
+};
+// Two samples' cells and weights.
+struct RefPos {
+    int j[2], i[2], k[2];
+    F2 xd, yd, zd;
+};
+
+// sample_ref's cell and weight along one axis, for two positions u: `inv` and
+// `n` divide by the extent and the dim.  The weight's sign is left to the
+// caller: rounding is symmetric, so its magnitude is the reference's.
+__device__ __forceinline__ F2 ref_axis(F2 u, float bmin, float extent, int dim, const FixedDiv &inv, const FixedDiv &n,
+                                       int (&cell)[2])
+{
+    float r0, r1;
+    f2_split(f2((float) dim) * inv(u + f2(-bmin)), r0, r1);
+    cell[0] = max(min((int) r0, dim - 2), 0);
+    cell[1] = max(min((int) r1, dim - 2), 0);
+    const F2 mu0 = n(f2((float) cell[0], (float) cell[1]) * f2(-extent));  // minus the cell's corner
+    return n(((u + f2(fabsf(bmin))) + mu0) * f2(extent));
+}
+
+__device__ __forceinline__ RefPos ref_pos(const DevBrick &b, const RefSampler &r, F2 x, F2 y, F2 z)
+{
+    RefPos p;
+    p.xd = ref_axis(x, b.bminx, b.w, b.nx, r.w, r.nx, p.j);
+    p.yd = ref_axis(y, b.bminy, b.h, b.ny, r.h, r.ny, p.i);
+    p.zd = ref_axis(z, b.bminz, b.d, b.nz, r.d, r.nz, p.k);
+    return p;
+}
+
+// The cell's voxels as loaded: from the corner-packed copy (an f32 copy holds
+// differences, which do not give the voxels back), or one by one.
+template <int DT> struct RefCell {
+    using E = typename VoxT<DT>::V4;
+    E lo, hi;
+};
+
+template <int DT>
+__device__ __forceinline__ RefCell<DT> ref_load(const DevBrick &b, int j, int i, int k)
+{
+    using V = typename VoxT<DT>::V4;
+    using T = typename VoxT<DT>::T;
+    RefCell<DT> c;
+    if (DT != IVR_F32 && b.quad) {
+        const unsigned qx = (unsigned) b.nx - 1u, qs = qx * ((unsigned) b.ny - 1u);
+        const V *e = reinterpret_cast<const V *>(b.quad) + ((unsigned) k * qs + (unsigned) i * qx + (unsigned) j);
+        c.lo = __ldg(e);
+        c.hi = __ldg(e + qs);
+    } else {
+        const unsigned row = (unsigned) b.nx, slab = row * (unsigned) b.ny;
+        const T *q = reinterpret_cast<const T *>(b.data) + ((unsigned) k * slab + (unsigned) i * row + (unsigned) j);
+        c.lo.x = __ldg(q);
+        c.lo.y = __ldg(q + 1);
+        c.lo.z = __ldg(q + row);
+        c.lo.w = __ldg(q + row + 1);
+        c.hi.x = __ldg(q + slab);
+        c.hi.y = __ldg(q + slab + 1);
+        c.hi.z = __ldg(q + slab + row);
+        c.hi.w = __ldg(q + slab + row + 1);
+    }
+    return c;
+}
+
+// sample_ref's blend, operation for operation (the x weight blends the +1
+// row)
+template <int DT>
+__device__ __forceinline__ float ref_interp(const RefCell<DT> &c, float xd, float yd, float zd)
+{
+    const float v000 = (float) c.lo.x, v010 = (float) c.lo.y, v100 = (float) c.lo.z, v110 = (float) c.lo.w;
+    const float v001 = (float) c.hi.x, v011 = (float) c.hi.y, v101 = (float) c.hi.z, v111 = (float) c.hi.w;
+    const float xe = 1.0f - xd, ye = 1.0f - yd, ze = 1.0f - zd;
+    const float c00 = v000 * xe + v100 * xd;
+    const float c10 = v010 * xe + v110 * xd;
+    const float c01 = v001 * xe + v101 * xd;
+    const float c11 = v011 * xe + v111 * xd;
+    const float c0 = c00 * ye + c10 * yd;
+    const float c1 = c01 * ye + c11 * yd;
+    return c0 * ze + c1 * zd;
+}
+
 __device__ __forceinline__ float lerpf(float a, float b, float t) { return fmaf(t, b - a, a); }
 
 // CONFIG sampler: trilinear with voxel values at cell corners (the
@@ -383,13 +558,100 @@ __device__ __forceinline__ float4 lut_at(const FrameDesc &f, int idx)
     return __ldg(f.lut + idx);
 }
 
+// One sample of a transfer function of transferfuncs.c:24-199, composited
+// into c = (r, g, b, a).
+template <int TF>
+__device__ __forceinline__ void ref_composite(const FrameDesc &f, float s, const float4 &e, float4 &c)
+{
+    const float myalpha = f.alpha;
+    if (TF == IVR_TF_MED) {  // transferfuncs.c:24-68
+        c.z = ((double) e.z < 0.8) ? fmaxf(e.z, c.z) : c.z;
+        c.y = ((double) e.y < 0.8) ? fmaxf(e.y, c.y) : c.y;
+        c.x = ((double) e.x < 0.8) ? fmaxf(e.x, c.x) : c.x;
+        c.w = e.w * myalpha;
+    } else if (TF == IVR_TF_BLEND) {  // transferfuncs.c:70-83
+        const float al = e.w;
+        c.z = al * e.z + (1.0f - al) * c.z;
+        c.y = al * e.y + (1.0f - al) * c.y;
+        c.x = al * e.x + (1.0f - al) * c.x;
+        c.w = al * myalpha;
+    } else if (TF == IVR_TF_SEISMIC2 || TF == IVR_TF_CHEM) {  // transferfuncs.c:109-168
+        const float al = e.w * myalpha;
+        const float oma = 1.0f - al;
+        c.z = oma * c.z + al * e.z;
+        c.y = oma * c.y + al * e.y;
+        c.x = oma * c.x + al * e.x;
+        c.w = al + oma * c.w;
+        if (c.w > 1.0f) c.w = 1.0f;
+    } else if (TF == IVR_TF_RGBBLEND) {  // transferfuncs.c:170-200
+        const unsigned u = __float_as_uint(s);
+        const float r = 1.0f / 255.0f * (float) ((u >> 24) & 0xff);
+        const float g = 1.0f / 255.0f * (float) ((u >> 16) & 0xff);
+        const float bl = 1.0f / 255.0f * (float) ((u >> 8) & 0xff);
+        const float al = myalpha;
+        const float oma = 1.0f - al;
+        c.z = oma * c.z + al * bl;
+        c.y = oma * c.y + al * g;
+        c.x = oma * c.x + al * r;
+        c.w = al + oma * c.w;
+        if (c.w > 1.0f) c.w = 1.0f;
+    } else {  // IVR_TF_SEISMIC, transferfuncs.c:86-107
+        c.z = ((double) e.z > 0.65 && e.z < 1.0f) ? 0.6f : c.z;
+        c.y = ((double) e.y > 0.65 && e.y < 1.0f) ? 0.0f : c.y;
+        c.x = ((double) e.x > 0.65 && e.x < 1.0f) ? 0.0f : c.x;
+        c.z = ((double) e.z > 0.5 && e.z < 0.65f) ? 0.9f : c.z;
+        c.y = ((double) e.y > 0.5 && e.y < 0.65f) ? 0.9f : c.y;
+        c.x = ((double) e.x > 0.5 && e.x < 0.65f) ? 0.9f : c.x;
+        c.z = ((double) e.z > 0.3 && e.z < 0.5f) ? 0.0f : c.z;
+        c.y = ((double) e.y > 0.3 && e.y < 0.5f) ? 0.0f : c.y;
+        c.x = ((double) e.x > 0.3 && e.x < 0.5f) ? 0.6f : c.x;
+        c.w = 1.0f * myalpha;
+    }
+}
+
 // raycast (ray.c:59-85) + getsamplesonray (ray.c:239-273) + one transfer
-// function of transferfuncs.c:24-199.  Samples are computed in the order the
-// transfer function consumes them (ascending or descending) instead of
-// being stored.  Returns (r, g, b, a).
+// function.  Samples are computed in the order the transfer function
+// consumes them (ascending or descending) instead of being stored, kRefPairs
+// pairs at a time with their loads in flight together.  Returns (r, g, b, a).
+// Bound by instruction issue (68% of the slots, 202 M warp instructions for
+// 128^3 u8 at 512x512): nine IEEE divisions a sample and up to 512 column
+// increments a pixel took 425 us; FixedDivs and shared increments 271; the
+// divisions of two samples packed, two pairs in flight, 254 (one pair 269).
+// 4, 6 and 8 blocks per SM instead of 5: 260, 265, 299.
+constexpr int kRefPairs = 2;        // pairs of samples per iteration
+constexpr int kRefBlocksPerSm = 5;  // resident blocks it is compiled for
+template <int TF> __device__ __forceinline__ constexpr bool ref_down()
+{
+    return TF == IVR_TF_SEISMIC2 || TF == IVR_TF_CHEM || TF == IVR_TF_RGBBLEND;
+}
+
+// the LUT entry of a sample: BLEND takes no lutoffset; lut_at clamps every
+// index (as SEISMIC2 and CHEM do)
+template <int TF>
+__device__ __forceinline__ float4 ref_entry(const FrameDesc &f, float s)
+{
+    if (TF == IVR_TF_RGBBLEND) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    return lut_at(f, (int) s - (TF == IVR_TF_BLEND ? 0 : f.lut_off));
+}
+
+// The ray's iend samples by sample_ref itself, one by one: rays on which
+// FixedDiv might round otherwise (ref_fast).
 template <int DT, int TF>
-__device__ float4 raycast_ref(const FrameDesc &f, const DevBrick &b, float dx, float dy, float dz,
-                              unsigned long long &nexec)
+__device__ __noinline__ float4 raycast_ref_general(const FrameDesc &f, const DevBrick &b, float dx, float dy, float dz,
+                                                   float tin, int iend)
+{
+    float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int n = 0; n < iend; n++) {
+        const float t = tin + ((float) (ref_down<TF>() ? iend - 1 - n : n) * f.step);
+        const float s = sample_ref<DT>(b, dx * t + f.origx, dy * t + f.origy, dz * t + f.origz);
+        ref_composite<TF>(f, s, ref_entry<TF>(f, s), c);
+    }
+    return c;
+}
+
+template <int DT, int TF>
+__device__ __forceinline__ float4 raycast_ref(const FrameDesc &f, const DevBrick &b, float dx, float dy, float dz,
+                                              unsigned long long &nexec)
 {
     float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float tin, tout;
@@ -399,70 +661,40 @@ __device__ float4 raycast_ref(const FrameDesc &f, const DevBrick &b, float dx, f
     if (f.max_samples > 0 && iend > f.max_samples) iend = f.max_samples;
     if (iend <= 0) return c;
     nexec += (unsigned long long) iend;
-    const float ox = f.origx, oy = f.origy, oz = f.origz;
-    const float myalpha = f.alpha;
-    auto sample = [&](int i) {
-        float t = tin + ((float) i * dt);
-        return sample_ref<DT>(b, dx * t + ox, dy * t + oy, dz * t + oz);
-    };
-    if (TF == IVR_TF_MED) {  // transferfuncs.c:24-68
-        for (int i = 0; i < iend; ++i) {
-            float4 e = lut_at(f, (int) sample(i) - f.lut_off);
-            c.z = ((double) e.z < 0.8) ? fmaxf(e.z, c.z) : c.z;
-            c.y = ((double) e.y < 0.8) ? fmaxf(e.y, c.y) : c.y;
-            c.x = ((double) e.x < 0.8) ? fmaxf(e.x, c.x) : c.x;
-            c.w = e.w * myalpha;
+    if (!ref_fast(f, b, dx, dy, dz, tin)) return raycast_ref_general<DT, TF>(f, b, dx, dy, dz, tin, iend);
+    const RefSampler rs(b);
+    for (int n = 0; n < iend; n += 2 * kRefPairs) {
+        RefPos p[kRefPairs];
+        RefCell<DT> v[2 * kRefPairs];
+#pragma unroll
+        for (int k = 0; k < kRefPairs; k++) {
+            // (past the last sample the last one again, not composited)
+            const int a = min(n + 2 * k, iend - 1), e = min(n + 2 * k + 1, iend - 1);
+            const float ta = tin + ((float) (ref_down<TF>() ? iend - 1 - a : a) * dt);
+            const float te = tin + ((float) (ref_down<TF>() ? iend - 1 - e : e) * dt);
+            p[k] = ref_pos(b, rs, f2(dx * ta + f.origx, dx * te + f.origx), f2(dy * ta + f.origy, dy * te + f.origy),
+                           f2(dz * ta + f.origz, dz * te + f.origz));
+#pragma unroll
+            for (int q = 0; q < 2; q++) v[2 * k + q] = ref_load<DT>(b, p[k].j[q], p[k].i[q], p[k].k[q]);
         }
-    } else if (TF == IVR_TF_BLEND) {  // transferfuncs.c:70-83 (no lutoffset)
-        for (int i = 0; i < iend; ++i) {
-            float4 e = lut_at(f, (int) sample(i));
-            float al = e.w;
-            c.z = al * e.z + (1.0f - al) * c.z;
-            c.y = al * e.y + (1.0f - al) * c.y;
-            c.x = al * e.x + (1.0f - al) * c.x;
-            c.w = al * myalpha;
+        float s[2 * kRefPairs];
+        float4 e[2 * kRefPairs];
+#pragma unroll
+        for (int k = 0; k < kRefPairs; k++) {
+            float xd[2], yd[2], zd[2];
+            f2_split(p[k].xd, xd[0], xd[1]);
+            f2_split(p[k].yd, yd[0], yd[1]);
+            f2_split(p[k].zd, zd[0], zd[1]);
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+                s[2 * k + q] = ref_interp<DT>(v[2 * k + q], fabsf(xd[q]), fabsf(yd[q]), fabsf(zd[q]));
         }
-    } else if (TF == IVR_TF_SEISMIC2 || TF == IVR_TF_CHEM) {  // transferfuncs.c:109-168
-        for (int i = iend - 1; i >= 0; i--) {
-            int idx = (int) sample(i) - f.lut_off;
-            if (idx < 0) idx = 0;
-            if (TF == IVR_TF_SEISMIC2 && idx > f.lut_n - 1) idx = f.lut_n - 1;
-            float4 e = lut_at(f, idx);
-            float al = e.w * myalpha;
-            float oma = 1.0f - al;
-            c.z = oma * c.z + al * e.z;
-            c.y = oma * c.y + al * e.y;
-            c.x = oma * c.x + al * e.x;
-            c.w = al + oma * c.w;
-            if (c.w > 1.0f) c.w = 1.0f;
-        }
-    } else if (TF == IVR_TF_RGBBLEND) {  // transferfuncs.c:170-200
-        for (int i = iend - 1; i >= 0; i--) {
-            unsigned u = __float_as_uint(sample(i));
-            float r = 1.0f / 255.0f * (float) ((u >> 24) & 0xff);
-            float g = 1.0f / 255.0f * (float) ((u >> 16) & 0xff);
-            float bl = 1.0f / 255.0f * (float) ((u >> 8) & 0xff);
-            float al = myalpha;
-            float oma = 1.0f - al;
-            c.z = oma * c.z + al * bl;
-            c.y = oma * c.y + al * g;
-            c.x = oma * c.x + al * r;
-            c.w = al + oma * c.w;
-            if (c.w > 1.0f) c.w = 1.0f;
-        }
-    } else {  // IVR_TF_SEISMIC, transferfuncs.c:86-107
-        for (int i = 0; i < iend; ++i) {
-            float4 e = lut_at(f, (int) sample(i) - f.lut_off);
-            c.z = ((double) e.z > 0.65 && e.z < 1.0f) ? 0.6f : c.z;
-            c.y = ((double) e.y > 0.65 && e.y < 1.0f) ? 0.0f : c.y;
-            c.x = ((double) e.x > 0.65 && e.x < 1.0f) ? 0.0f : c.x;
-            c.z = ((double) e.z > 0.5 && e.z < 0.65f) ? 0.9f : c.z;
-            c.y = ((double) e.y > 0.5 && e.y < 0.65f) ? 0.9f : c.y;
-            c.x = ((double) e.x > 0.5 && e.x < 0.65f) ? 0.9f : c.x;
-            c.z = ((double) e.z > 0.3 && e.z < 0.5f) ? 0.0f : c.z;
-            c.y = ((double) e.y > 0.3 && e.y < 0.5f) ? 0.0f : c.y;
-            c.x = ((double) e.x > 0.3 && e.x < 0.5f) ? 0.6f : c.x;
-            c.w = 1.0f * myalpha;
+#pragma unroll
+        for (int k = 0; k < 2 * kRefPairs; k++) e[k] = ref_entry<TF>(f, s[k]);
+#pragma unroll
+        for (int k = 0; k < 2 * kRefPairs; k++) {
+            if (n + k >= iend) break;
+            ref_composite<TF>(f, s[k], e[k], c);
         }
     }
     return c;
@@ -801,26 +1033,43 @@ __device__ __forceinline__ void pixel_of(const FrameDesc &f, int &i, int &j, int
 }
 
 template <int DT, int TF>
-__global__ void __launch_bounds__(kThreads) march_ref_kernel(const __grid_constant__ FrameDesc f, float4 *out32,
+__global__ void __launch_bounds__(kThreads, kRefBlocksPerSm) march_ref_kernel(const __grid_constant__ FrameDesc f, float4 *out32,
                                                              uchar4 *out8)
 {
+    // Each brick casts its own ray with the sequential column increments of
+    // createlocalimage (main.c:986-999): a chain of up to the window's width
+    // of additions, each rounded, so nothing shorter gives its value.  Per
+    // brick, row and component one lane walks the chain to the block's first
+    // column (s_dir); the pixels add at most kBlockX more.
+    __shared__ float s_dir[kMaxBricks][kBlockY][3];
+    const int j0 = f.out_x + (int) blockIdx.x * kBlockX, i0 = f.out_y + (int) blockIdx.y * kBlockY;
+    for (int q = threadIdx.x >> 5; q < f.nb; q += kThreads / 32) {
+        const DevBrick &b = f.b[q];
+        const int lane = threadIdx.x & 31, row = lane / 3, comp = lane - 3 * row;
+        if (row >= kBlockY || (f.single >= 0 && q != f.single)) continue;
+        if (j0 + kBlockX <= b.jstrt || j0 >= b.jstop || i0 + kBlockY <= b.istrt || i0 >= b.istop) continue;
+        const float fi = (float) (i0 + row - b.istrt);
+        float dir = comp == 0 ? b.dir0x + f.incrix * fi : comp == 1 ? b.dir0y + f.incriy * fi : b.dir0z + f.incriz * fi;
+        const float incr = comp == 0 ? f.incrjx : comp == 1 ? f.incrjy : f.incrjz;
+        for (int c = b.jstrt; c < j0; c++) dir += incr;
+        s_dir[q][row][comp] = dir;
+    }
+    __syncthreads();
     int i, j, oi, oj;
     pixel_of(f, i, j, oi, oj);
     const bool inside = oj < f.out_w && oi < f.out_h;
     float4 d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     unsigned long long nexec = 0;
     if (inside && i < f.vh && j < f.vw) {
-        // far -> near over of per-brick colours; each brick casts its own ray
-        // with the sequential column increments of createlocalimage
-        // (main.c:986-999)
+        // far -> near over of per-brick colours
         for (int s = f.nb - 1; s >= 0; s--) {
             const int k = f.order[s];
             if (f.single >= 0 && k != f.single) continue;
             const DevBrick &b = f.b[k];
             if (!in_rect(b, i, j)) continue;
-            const float fi = (float) (i - b.istrt);
-            float dx = b.dir0x + f.incrix * fi, dy = b.dir0y + f.incriy * fi, dz = b.dir0z + f.incriz * fi;
-            for (int c = b.jstrt; c <= j; c++) {
+            const float *dir = s_dir[k][i - i0];
+            float dx = dir[0], dy = dir[1], dz = dir[2];
+            for (int c = max(b.jstrt, j0); c <= j; c++) {
                 dx += f.incrjx;
                 dy += f.incrjy;
                 dz += f.incrjz;
