@@ -24,17 +24,6 @@ int grid_for(long long n, int threads, int per_sm = 8)
     return (int) (g < cap ? (g < 1 ? 1 : g) : cap);
 }
 
-template <typename T> __device__ __forceinline__ float tof(T v) { return (float) v; }
-
-__device__ __forceinline__ float load_any(const void *p, int dtype, long long i)
-{
-    switch (dtype) {
-    case IVR_U8: return (float) __ldg(reinterpret_cast<const uint8_t *>(p) + i);
-    case IVR_U16: return (float) __ldg(reinterpret_cast<const uint16_t *>(p) + i);
-    default: return __ldg(reinterpret_cast<const float *>(p) + i);
-    }
-}
-
 __global__ void byteswap16_kernel(uint16_t *p, long long n)
 {
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x)
@@ -50,16 +39,24 @@ __global__ void byteswap32_kernel(uint32_t *p, long long n)
 
 // readfromfile (main.c:1254-1265): brick [sz..sz+ld) x [sy..sy+lh) x
 // [sx..sx+lw) of the global volume into a dense [ld][lh][lw] array.
+// A warp copies whole rows, four 32-voxel pieces in flight; HBM-bound.
 template <typename T>
-__global__ void gather_kernel(const T *__restrict__ src, int gw, int gh, T *__restrict__ dst, int sx, int sy,
-                              int sz, int lw, int lh, long long n)
+__global__ void __launch_bounds__(256) gather_kernel(const T *__restrict__ src, int gw, int gh, T *__restrict__ dst,
+                                                     int sx, int sy, int sz, int lw, int lh, long long rows)
 {
-    for (long long o = blockIdx.x * (long long) blockDim.x + threadIdx.x; o < n; o += (long long) gridDim.x * blockDim.x) {
-        int x = (int) (o % lw);
-        long long r = o / lw;
-        int y = (int) (r % lh);
-        int z = (int) (r / lh);
-        dst[o] = src[((long long) (sz + z) * gh + (sy + y)) * gw + (sx + x)];
+    const int lane = threadIdx.x & 31;
+    const long long r = (long long) blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (r >= rows) return;
+    const int y = (int) (r % lh), z = (int) (r / lh);
+    const T *p = src + ((long long) (sz + z) * gh + (sy + y)) * gw + sx;
+    T *q = dst + r * lw;
+    for (int x = lane; x < lw; x += 128) {
+        T v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = x + 32 * u < lw ? __ldg(p + x + 32 * u) : T(0);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (x + 32 * u < lw) q[x + 32 * u] = v[u];
     }
 }
 
@@ -281,39 +278,168 @@ __global__ void hist_global_kernel(const T *__restrict__ data, long long n, MinA
     if ((threadIdx.x & 31) == 0 && zero) atomicAdd(&hist[0], zero);
 }
 
-// Macrocell min/max: with edge `cell`, cell (cx,cy,cz) spans voxels
-// [c*cell, min(c*cell+cell, n-1)] per axis -- its voxel cells plus the +1
-// layer a trilinear sample in the cell also reads.  One block per cell.
-__global__ void macrocell_kernel(const void *data, int dtype, int nx, int ny, int nz, int cell, float *mc, int mcx,
-                                 int mcy)
+// Macrocell min/max: with edge c = 2^cs, cell (cx,cy,cz) spans voxels
+// [c*cx, min(c*cx+c, n-1)] per axis -- its voxel cells plus the +1 layer a
+// trilinear sample in the cell also reads.  HBM-bound: the volume is read
+// once, (c+1)^2/c^2 of it with the layers that neighbouring cells share
+// (those mostly from L2).  A block takes the cells over a segment of kCols
+// columns: its 8 warps share the (c+1)^2 rows of the segment, each lane
+// keeping the min and max of its columns over its warp's rows, and the rows'
+// results meet in shared memory.  One block per cell with two divisions per
+// voxel took 3.5 ms for 1024^3 u16 voxels (0.6 TB/s).
+// VEC: rows start on 16 bytes and a lane's columns are one 16-byte load,
+// integer voxels compared as packed lanes; otherwise they are 4 columns 32
+// apart.
+constexpr int kMcWarps = 8;
+template <typename T, bool VEC> struct McTile {
+    static constexpr int kPer = VEC ? kVec<T> : 4;  // columns a lane
+    static constexpr int kCols = 32 * kPer;
+    T lo[kMcWarps][kCols], hi[kMcWarps][kCols];
+    T xlo[kMcWarps], xhi[kMcWarps];  // the column after the segment
+};
+template <typename T> __device__ __forceinline__ T vmin_of(T a, T b) { return a < b ? a : b; }
+template <typename T> __device__ __forceinline__ T vmax_of(T a, T b) { return a > b ? a : b; }
+template <> __device__ __forceinline__ float vmin_of(float a, float b) { return fminf(a, b); }
+template <> __device__ __forceinline__ float vmax_of(float a, float b) { return fmaxf(a, b); }
+template <typename T> __device__ __forceinline__ T vtop() { return (T) ~(T) 0; }
+template <> __device__ __forceinline__ float vtop<float>() { return FLT_MAX; }
+template <typename T> __device__ __forceinline__ T vbottom() { return 0; }
+template <> __device__ __forceinline__ float vbottom<float>() { return -FLT_MAX; }
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(32 * kMcWarps) macrocell_kernel(const T *__restrict__ data, int nx, int ny, int nz,
+                                                                  int cs, float *mc, int mcx, int mcy, int nseg)
 {
-    const int cid = blockIdx.x;
-    const int cx = cid % mcx, cy = (cid / mcx) % mcy, cz = cid / (mcx * mcy);
-    const int x0 = cx * cell, y0 = cy * cell, z0 = cz * cell;
-    const int x1 = min(x0 + cell, nx - 1), y1 = min(y0 + cell, ny - 1), z1 = min(z0 + cell, nz - 1);
-    const int ex = x1 - x0 + 1, ey = y1 - y0 + 1, ez = z1 - z0 + 1;
-    float lo = FLT_MAX, hi = -FLT_MAX;
-    const int tot = ex * ey * ez;
-    for (int t = threadIdx.x; t < tot; t += blockDim.x) {
-        int x = t % ex, r = t / ex;
-        int y = r % ey, z = r / ey;
-        float v = load_any(data, dtype, ((long long) (z0 + z) * ny + (y0 + y)) * nx + (x0 + x));
-        lo = fminf(lo, v);
-        hi = fmaxf(hi, v);
+    using Tile = McTile<T, VEC>;
+    constexpr int kPer = Tile::kPer, kCols = Tile::kCols;
+    __shared__ __align__(16) Tile s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = 1 << cs;
+    const unsigned seg = blockIdx.x % nseg, rest = blockIdx.x / nseg;
+    const int cy = (int) (rest % mcy), cz = (int) (rest / mcy), xb = (int) seg * kCols;
+    const int y0 = cy << cs, z0 = cz << cs;
+    const int ey = min(y0 + c, ny - 1) - y0 + 1, ez = min(z0 + c, nz - 1) - z0 + 1, rows = ey * ez;
+    auto row = [&](int r) { return data + ((long long) (z0 + r / ey) * ny + (y0 + r % ey)) * nx; };
+    // this lane's columns over the warp's rows
+    MinMaxAcc<T> acc[4];           // VEC: one per 32-bit word of the load
+    T lo[kPer], hi[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+        lo[u] = vtop<T>();
+        hi[u] = vbottom<T>();
     }
+    if constexpr (VEC) {
+        const int x = xb + lane * kPer;  // nx is a multiple of kPer
+        if (x < nx) {
+            for (int r = warp; r < rows; r += 4 * kMcWarps) {
+                uint4 v[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++)  // past the last row: the last one again
+                    v[u] = __ldg(reinterpret_cast<const uint4 *>(row(min(r + u * kMcWarps, rows - 1)) + x));
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    acc[0].word(v[u].x);
+                    acc[1].word(v[u].y);
+                    acc[2].word(v[u].z);
+                    acc[3].word(v[u].w);
+                }
+            }
+        }
+        uint4 l, h;
+        if constexpr (sizeof(T) == 4) {
+            l = make_uint4(__float_as_uint(acc[0].lo), __float_as_uint(acc[1].lo), __float_as_uint(acc[2].lo), __float_as_uint(acc[3].lo));
+            h = make_uint4(__float_as_uint(acc[0].hi), __float_as_uint(acc[1].hi), __float_as_uint(acc[2].hi), __float_as_uint(acc[3].hi));
+        } else {
+            l = make_uint4(acc[0].lo, acc[1].lo, acc[2].lo, acc[3].lo);
+            h = make_uint4(acc[0].hi, acc[1].hi, acc[2].hi, acc[3].hi);
+        }
+        *reinterpret_cast<uint4 *>(&s.lo[warp][lane * kPer]) = l;
+        *reinterpret_cast<uint4 *>(&s.hi[warp][lane * kPer]) = h;
+    } else {
+        for (int r = warp; r < rows; r += 2 * kMcWarps) {
+            const T *p = row(r), *q = row(min(r + kMcWarps, rows - 1));
+            T v[2][kPer];
+#pragma unroll
+            for (int u = 0; u < kPer; u++) {  // past the last column: the last one again
+                const int x = min(xb + lane + 32 * u, nx - 1);
+                v[0][u] = __ldg(p + x);
+                v[1][u] = __ldg(q + x);
+            }
+#pragma unroll
+            for (int u = 0; u < kPer; u++) {
+                lo[u] = vmin_of(lo[u], vmin_of(v[0][u], v[1][u]));
+                hi[u] = vmax_of(hi[u], vmax_of(v[0][u], v[1][u]));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            s.lo[warp][lane + 32 * u] = lo[u];
+            s.hi[warp][lane + 32 * u] = hi[u];
+        }
+    }
+    T xl = vtop<T>(), xh = vbottom<T>();
+    if (xb + kCols < nx)
+        for (int r = warp + lane * kMcWarps; r < rows; r += 32 * kMcWarps) {
+            const T v = __ldg(row(r) + xb + kCols);
+            xl = vmin_of(xl, v);
+            xh = vmax_of(xh, v);
+        }
     for (int o = 16; o > 0; o >>= 1) {
-        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        xl = vmin_of(xl, (T) __shfl_xor_sync(0xffffffffu, xl, o));
+        xh = vmax_of(xh, (T) __shfl_xor_sync(0xffffffffu, xh, o));
     }
-    __shared__ float slo[32], shi[32];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) { slo[w] = lo; shi[w] = hi; }
+    if (lane == 0) {
+        s.xlo[warp] = xl;
+        s.xhi[warp] = xh;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < (int) (blockDim.x >> 5); k++) { lo = fminf(lo, slo[k]); hi = fmaxf(hi, shi[k]); }
-        mc[2 * cid] = lo;
-        mc[2 * cid + 1] = hi;
+    // the warps' rows together: thread t owns columns t, t + 256, ...
+    for (int x = threadIdx.x; x < kCols; x += 32 * kMcWarps) {
+        T l = s.lo[0][x], h = s.hi[0][x];
+#pragma unroll
+        for (int w = 1; w < kMcWarps; w++) {
+            l = vmin_of(l, s.lo[w][x]);
+            h = vmax_of(h, s.hi[w][x]);
+        }
+        s.lo[0][x] = l;
+        s.hi[0][x] = h;
     }
+    if (threadIdx.x == 0)
+        for (int w = 1; w < kMcWarps; w++) {
+            s.xlo[0] = vmin_of(s.xlo[0], s.xlo[w]);
+            s.xhi[0] = vmax_of(s.xhi[0], s.xhi[w]);
+        }
+    __syncthreads();
+    // a cell's c columns (c divides 32) and the next one
+    for (int x = threadIdx.x; x < kCols; x += 32 * kMcWarps) {
+        T l = s.lo[0][x], h = s.hi[0][x];
+        for (int o = c >> 1; o > 0; o >>= 1) {
+            l = vmin_of(l, (T) __shfl_xor_sync(0xffffffffu, l, o));
+            h = vmax_of(h, (T) __shfl_xor_sync(0xffffffffu, h, o));
+        }
+        const int cx = (xb + x) >> cs;
+        if ((x & (c - 1)) == 0 && cx < mcx) {
+            const bool last = x + c == kCols;
+            l = vmin_of(l, last ? s.xlo[0] : s.lo[0][x + c]);
+            h = vmax_of(h, last ? s.xhi[0] : s.hi[0][x + c]);
+            float *o = mc + 2 * (((long long) cz * mcy + cy) * mcx + cx);
+            *reinterpret_cast<float2 *>(o) = make_float2((float) l, (float) h);
+        }
+    }
+}
+
+template <typename T>
+cudaError_t macrocells_dt(const T *data, int nx, int ny, int nz, int cell, float *mc, int mcx, int mcy, int mcz,
+                          cudaStream_t s)
+{
+    int cs = 0;
+    while ((1 << cs) < cell) cs++;
+    const bool vec = (long long) nx * sizeof(T) % 16 == 0 && reinterpret_cast<uintptr_t>(data) % 16 == 0;
+    const int cols = vec ? McTile<T, true>::kCols : McTile<T, false>::kCols;
+    const int nseg = (mcx * cell + cols - 1) / cols;
+    const unsigned grid = (unsigned) ((long long) nseg * mcy * mcz);
+    if (vec) macrocell_kernel<T, true><<<grid, 32 * kMcWarps, 0, s>>>(data, nx, ny, nz, cs, mc, mcx, mcy, nseg);
+    else macrocell_kernel<T, false><<<grid, 32 * kMcWarps, 0, s>>>(data, nx, ny, nz, cs, mc, mcx, mcy, nseg);
+    return cudaGetLastError();
 }
 
 // A cell is transparent when no LUT entry its samples can index has
@@ -608,11 +734,11 @@ cudaError_t launch_gather_brick(const void *src, int gw, int gh, int gd, void *d
                                 int lh, int ld, int elem, cudaStream_t s)
 {
     (void) gd;
-    long long n = (long long) lw * lh * ld;
-    int g = grid_for(n, 256);
-    if (elem == 1) gather_kernel<uint8_t><<<g, 256, 0, s>>>((const uint8_t *) src, gw, gh, (uint8_t *) dst, sx, sy, sz, lw, lh, n);
-    else if (elem == 2) gather_kernel<uint16_t><<<g, 256, 0, s>>>((const uint16_t *) src, gw, gh, (uint16_t *) dst, sx, sy, sz, lw, lh, n);
-    else gather_kernel<uint32_t><<<g, 256, 0, s>>>((const uint32_t *) src, gw, gh, (uint32_t *) dst, sx, sy, sz, lw, lh, n);
+    const long long rows = (long long) lh * ld;
+    const unsigned g = (unsigned) ((rows + 7) / 8);
+    if (elem == 1) gather_kernel<<<g, 256, 0, s>>>((const uint8_t *) src, gw, gh, (uint8_t *) dst, sx, sy, sz, lw, lh, rows);
+    else if (elem == 2) gather_kernel<<<g, 256, 0, s>>>((const uint16_t *) src, gw, gh, (uint16_t *) dst, sx, sy, sz, lw, lh, rows);
+    else gather_kernel<<<g, 256, 0, s>>>((const uint32_t *) src, gw, gh, (uint32_t *) dst, sx, sy, sz, lw, lh, rows);
     return cudaGetLastError();
 }
 
@@ -631,8 +757,11 @@ cudaError_t launch_histogram(const void *data, int dtype, long long n, float mn,
 cudaError_t launch_macrocells(const void *data, int dtype, int nx, int ny, int nz, int cell, float *mc, int mcx,
                               int mcy, int mcz, cudaStream_t s)
 {
-    macrocell_kernel<<<mcx * mcy * mcz, 128, 0, s>>>(data, dtype, nx, ny, nz, cell, mc, mcx, mcy);
-    return cudaGetLastError();
+    switch (dtype) {
+    case IVR_U8: return macrocells_dt((const uint8_t *) data, nx, ny, nz, cell, mc, mcx, mcy, mcz, s);
+    case IVR_U16: return macrocells_dt((const uint16_t *) data, nx, ny, nz, cell, mc, mcx, mcy, mcz, s);
+    default: return macrocells_dt((const float *) data, nx, ny, nz, cell, mc, mcx, mcy, mcz, s);
+    }
 }
 
 cudaError_t launch_empty_flags(const float *mc, int mcx, int mcy, int mcz, const int *nzprefix, const double *aprefix,
@@ -702,26 +831,45 @@ cudaError_t launch_gradient(const void *data, int dtype, int w, int h, int d, fl
     return cudaGetLastError();
 }
 
+// Corner-packed copy; bound by its stores (4x the brick).  A warp takes 32
+// elements of a row and walks kQuadRows rows, each voxel row loaded once for
+// the two element rows it belongs to.  With a 64-bit division per index and
+// an element a thread it took 4.9 ms for 1024^3 u16 voxels (2.2 TB/s).
+constexpr int kQuadRows = 4;
 template <typename T, typename V>
-__global__ void quad_kernel(const T *src, int nx, int ny, int nz, V *dst)
+__global__ void __launch_bounds__(256) quad_kernel(const T *__restrict__ src, int nx, int ny, V *__restrict__ dst,
+                                                   unsigned bx, unsigned by)
 {
-    const long long qx = nx - 1, qy = ny - 1, n = qx * qy * nz;
-    for (long long e = blockIdx.x * (long long) blockDim.x + threadIdx.x; e < n;
-         e += (long long) gridDim.x * blockDim.x) {
-        const long long j = e % qx, r = e / qx, i = r % qy, k = r / qy;
-        const T *p = src + (k * ny + i) * nx + j;
+    const int qx = nx - 1, qy = ny - 1;
+    const unsigned r = blockIdx.x / bx;
+    const int j = (int) (blockIdx.x % bx) * 32 + (threadIdx.x & 31);
+    const int i0 = ((int) (r % by) * 8 + (int) (threadIdx.x >> 5)) * kQuadRows;
+    const long long k = r / by;
+    if (j >= qx || i0 >= qy) return;
+    const T *p = src + (k * ny + i0) * nx + j;
+    V *q = dst + (k * qy + i0) * qx + j;
+    T a[kQuadRows + 1], b[kQuadRows + 1];
+#pragma unroll
+    for (int u = 0; u <= kQuadRows; u++) {  // past the last row: the last one again
+        const T *row = p + (long long) min(u, qy - i0) * nx;
+        a[u] = __ldg(row);
+        b[u] = __ldg(row + 1);
+    }
+#pragma unroll
+    for (int u = 0; u < kQuadRows; u++) {
+        if (i0 + u >= qy) break;
         V v;
-        v.x = p[0];
-        v.y = p[1];
-        v.z = p[nx];
-        v.w = p[nx + 1];
+        v.x = a[u];
+        v.y = b[u];
+        v.z = a[u + 1];
+        v.w = b[u + 1];
         if constexpr (sizeof(T) == sizeof(float)) {
             if (kQuadDelta) {  // the sampler's x-lerp differences, rounded as it rounds them
-                v.y = p[1] - p[0];
-                v.w = p[nx + 1] - p[nx];
+                v.y = b[u] - a[u];
+                v.w = b[u + 1] - a[u + 1];
             }
         }
-        dst[e] = v;
+        q[(long long) u * qx] = v;
     }
 }
 
@@ -732,12 +880,12 @@ size_t quad_bytes(int dtype, int nx, int ny, int nz)
 
 cudaError_t launch_quads(const void *data, int dtype, int nx, int ny, int nz, void *quad, cudaStream_t s)
 {
-    const long long n = (long long) (nx - 1) * (ny - 1) * nz;
-    const int grid = grid_for(n, 256);
+    const unsigned bx = (unsigned) (nx - 1 + 31) / 32, by = (unsigned) (ny - 1 + 8 * kQuadRows - 1) / (8 * kQuadRows);
+    const unsigned grid = (unsigned) ((unsigned long long) bx * by * nz);
     switch (dtype) {
-    case IVR_U8: quad_kernel<<<grid, 256, 0, s>>>((const uint8_t *) data, nx, ny, nz, (uchar4 *) quad); break;
-    case IVR_U16: quad_kernel<<<grid, 256, 0, s>>>((const uint16_t *) data, nx, ny, nz, (ushort4 *) quad); break;
-    case IVR_F32: quad_kernel<<<grid, 256, 0, s>>>((const float *) data, nx, ny, nz, (float4 *) quad); break;
+    case IVR_U8: quad_kernel<<<grid, 256, 0, s>>>((const uint8_t *) data, nx, ny, (uchar4 *) quad, bx, by); break;
+    case IVR_U16: quad_kernel<<<grid, 256, 0, s>>>((const uint16_t *) data, nx, ny, (ushort4 *) quad, bx, by); break;
+    case IVR_F32: quad_kernel<<<grid, 256, 0, s>>>((const float *) data, nx, ny, (float4 *) quad, bx, by); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
