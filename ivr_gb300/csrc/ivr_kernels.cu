@@ -794,38 +794,52 @@ cudaError_t launch_dist_transform(uint8_t *dist, int mcx, int mcy, int mcz, cuda
 // Per-voxel gradient (gradient3d, restated as intended): per axis a halved
 // central difference inside and a halved one-sided difference on the
 // faces, times the unit spacing; w = |(x, y, z)| as mag3f computes it.
+// HBM-bound: the volume read once, 16 bytes written per voxel.  A thread
+// walks kGradRows rows down its column with the rows around it in registers;
+// the x and z neighbours come from L1 and L2.  512x512x384 f32 voxels: 560 us
+// with three 64-bit divisions per voxel; 332 us (6.1 TB/s) with 4 rows of 128
+// or 256 columns; 1, 2, 8 rows 461, 376, 340; 16 voxels up a z column instead,
+// whose stores touch 16 slabs at a time, 490.
+constexpr int kGradRows = 4, kGradColumns = 128;
 template <typename T>
-__device__ __forceinline__ float grad_axis(const T *v, long long o, int c, int n, long long stride)
+__global__ void __launch_bounds__(256) gradient_kernel(const T *__restrict__ vol, int w, int h, int d,
+                                                       float4 *__restrict__ out, unsigned bx, unsigned by)
 {
-    if (c == 0) return ((float) v[o + stride] - (float) v[o]) / 2.0f * 1.0f;
-    if (c == n - 1) return ((float) v[o] - (float) v[o - stride]) / 2.0f * 1.0f;
-    return ((float) v[o + stride] - (float) v[o - stride]) / 2.0f * 1.0f;
-}
-
-template <typename T>
-__global__ void gradient_kernel(const T *vol, int w, int h, int d, float4 *out)
-{
-    const long long n = (long long) w * h * d;
-    for (long long o = blockIdx.x * (long long) blockDim.x + threadIdx.x; o < n;
-         o += (long long) gridDim.x * blockDim.x) {
-        const int j = (int) (o % w);
-        const long long r = o / w;
-        const int i = (int) (r % h), k = (int) (r / h);
-        const float x = grad_axis(vol, o, j, w, 1);
-        const float y = grad_axis(vol, o, i, h, w);
-        const float z = grad_axis(vol, o, k, d, (long long) w * h);
-        out[o] = make_float4(x, y, z, sqrtf(x * x + y * y + z * z));
+    const unsigned r = blockIdx.x / bx;
+    const int j = (int) (blockIdx.x % bx * blockDim.x + threadIdx.x);
+    const int i0 = (int) (r % by * blockDim.y + threadIdx.y) * kGradRows, i1 = min(i0 + kGradRows, h);
+    const int k = (int) (r / by);
+    if (j >= w || i0 >= h) return;
+    const long long slab = (long long) w * h;
+    const T *p = vol + k * slab + (long long) i0 * w + j;
+    float4 *q = out + k * slab + (long long) i0 * w + j;
+    // offsets of the neighbours each difference takes
+    const int xl = j > 0 ? -1 : 0, xh = j < w - 1 ? 1 : 0;
+    const long long zl = k > 0 ? -slab : 0, zh = k < d - 1 ? slab : 0;
+    float below = (float) __ldg(i0 > 0 ? p - w : p), here = (float) __ldg(p);
+#pragma unroll
+    for (int u = 0; u < kGradRows; u++, p += w, q += w) {
+        if (i0 + u >= i1) break;
+        const float above = i0 + u < h - 1 ? (float) __ldg(p + w) : here;
+        const float x = ((float) __ldg(p + xh) - (float) __ldg(p + xl)) / 2.0f;
+        const float y = (above - below) / 2.0f;
+        const float z = ((float) __ldg(p + zh) - (float) __ldg(p + zl)) / 2.0f;
+        *q = make_float4(x, y, z, sqrtf(x * x + y * y + z * z));
+        below = here;
+        here = above;
     }
 }
 
 cudaError_t launch_gradient(const void *data, int dtype, int w, int h, int d, float4 *out, cudaStream_t s)
 {
-    const long long n = (long long) w * h * d;
-    const int grid = grid_for(n, 256);
+    const unsigned tx = (unsigned) std::min(kGradColumns, (w + 31) / 32 * 32);
+    const dim3 block(tx, 256 / tx);
+    const unsigned bx = (w + tx - 1) / tx, by = (h + block.y * kGradRows - 1) / (block.y * kGradRows);
+    const unsigned grid = (unsigned) ((unsigned long long) bx * by * d);
     switch (dtype) {
-    case IVR_U8: gradient_kernel<<<grid, 256, 0, s>>>((const uint8_t *) data, w, h, d, out); break;
-    case IVR_U16: gradient_kernel<<<grid, 256, 0, s>>>((const uint16_t *) data, w, h, d, out); break;
-    case IVR_F32: gradient_kernel<<<grid, 256, 0, s>>>((const float *) data, w, h, d, out); break;
+    case IVR_U8: gradient_kernel<<<grid, block, 0, s>>>((const uint8_t *) data, w, h, d, out, bx, by); break;
+    case IVR_U16: gradient_kernel<<<grid, block, 0, s>>>((const uint16_t *) data, w, h, d, out, bx, by); break;
+    case IVR_F32: gradient_kernel<<<grid, block, 0, s>>>((const float *) data, w, h, d, out, bx, by); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
