@@ -574,6 +574,22 @@ __device__ __forceinline__ unsigned q8k(float v)
     return (unsigned) ((255ull * m + (1ull << (s - 1))) >> s);
 }
 
+// HBM-bound; four floats in, one 32-bit word out per step where the buffers
+// allow it (a float a thread with single-byte stores took 17.7 us for
+// 1920x1080 RGBA, 2.3 TB/s), two steps in flight.
+__global__ void __launch_bounds__(256) quantize4_kernel(const float4 *__restrict__ in, uchar4 *__restrict__ out,
+                                                        long long n4)
+{
+    const long long stride = (long long) gridDim.x * blockDim.x;
+    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n4; i += 2 * stride) {
+        const bool two = i + stride < n4;
+        const float4 a = __ldg(in + i), b = two ? __ldg(in + i + stride) : a;
+        out[i] = make_uchar4(q8k(a.x), q8k(a.y), q8k(a.z), q8k(a.w));
+        if (two) out[i + stride] = make_uchar4(q8k(b.x), q8k(b.y), q8k(b.z), q8k(b.w));
+    }
+}
+
+// unaligned buffers, and the last n % 4 floats of the others
 __global__ void quantize_kernel(const float *__restrict__ in, uint8_t *__restrict__ out, long long n)
 {
     for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x)
@@ -913,7 +929,10 @@ cudaError_t launch_composite(float *dst, const float *src, int num, long long np
 
 cudaError_t launch_quantize(const float *in, uint8_t *out, long long n, cudaStream_t s)
 {
-    quantize_kernel<<<grid_for(n, 256), 256, 0, s>>>(in, out, n);
+    const bool vec = reinterpret_cast<uintptr_t>(in) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 4 == 0;
+    const long long n4 = vec ? n / 4 : 0;
+    if (n4 > 0) quantize4_kernel<<<grid_for((n4 + 1) / 2, 256), 256, 0, s>>>((const float4 *) in, (uchar4 *) out, n4);
+    if (n > 4 * n4) quantize_kernel<<<grid_for(n - 4 * n4, 256), 256, 0, s>>>(in + 4 * n4, out + 4 * n4, n - 4 * n4);
     return cudaGetLastError();
 }
 
