@@ -37,6 +37,11 @@ struct ivr_mlp {
     int *d_status = nullptr;  // tensor-core status word (kMlpTcTimeout): training, inference, grids
     unsigned long long *d_counts = nullptr;
     cudaEvent_t scratch_ev = nullptr;  // after the last use of d_knots
+    // training workspaces (ivr_mlp_train)
+    float *d_c12 = nullptr;
+    long long c12_cap = 0;
+    void *h_pinned = nullptr;
+    size_t pinned_bytes = 0;
 };
 
 namespace {
@@ -261,6 +266,8 @@ int ivr_mlp_free(ivr_mlp *m)
     dev_free(c, m->d_status, sizeof(int));
     dev_free(c, m->d_counts, 2 * sizeof(unsigned long long));
     if (m->scratch_ev) cudaEventDestroy(m->scratch_ev);
+    dev_free(c, m->d_c12, (size_t) m->c12_cap * sizeof(float));
+    cudaFreeHost(m->h_pinned);
     delete m;
     return IVR_OK;
 }
@@ -476,11 +483,30 @@ int ivr_mlp_train(ivr_mlp *m, int epochs, int batch_rows, float lr, float wneg, 
     const long long nb = (m->n + batch_rows - 1) / batch_rows;
     int rc = grow(c, (void **) &m->d_loss, &m->loss_cap, nb, sizeof(float), 0);
     if (rc) return rc;
-    // the Adam bias corrections of an epoch's steps, device-resident so that
-    // one captured epoch replays with each epoch's values
-    float *d_c12 = nullptr;
-    rc = dev_alloc(c, sizeof(float) * 2 * (size_t) nb, (void **) &d_c12);
+    // Workspaces of the epochs, kept with the predictor.  On the device: the
+    // Adam bias corrections of an epoch's steps, so that one captured epoch
+    // replays with each epoch's values.  Page-locked, in one block: the epochs'
+    // row orders (the host shuffles the next epoch's while the device trains
+    // on the current one; one buffer if there is no next), the epoch's bias
+    // corrections and its losses, so that no copy of an epoch waits for the
+    // host or the host for the device before the shuffle is done.
+    rc = grow(c, (void **) &m->d_c12, &m->c12_cap, 2 * nb, sizeof(float), 0);
     if (rc) return rc;
+    const size_t n = (size_t) m->n;
+    const int norders = epochs > 1 ? 2 : 1;
+    const size_t host_bytes = sizeof(float) * 3 * (size_t) nb + sizeof(int) * n * (size_t) norders;
+    cudaError_t e = cudaDeviceSynchronize();
+    if (e == cudaSuccess && m->pinned_bytes < host_bytes) {
+        cudaFreeHost(m->h_pinned);
+        m->h_pinned = nullptr;
+        m->pinned_bytes = 0;
+        e = cudaHostAlloc(&m->h_pinned, host_bytes, 0);
+        if (e == cudaSuccess) m->pinned_bytes = host_bytes;
+    }
+    if (e != cudaSuccess) return cuda_fail(c, e, "training order buffers");
+    float *d_c12 = m->d_c12, *c12 = (float *) m->h_pinned, *losses = c12 + 2 * nb;
+    int *order[2] = {(int *) (losses + nb), nullptr};
+    if (norders > 1) order[1] = order[0] + n;
     struct Graph {
         cudaStream_t s = nullptr;
         cudaGraph_t g = nullptr;
@@ -492,64 +518,41 @@ int ivr_mlp_train(ivr_mlp *m, int epochs, int batch_rows, float lr, float wneg, 
             if (s) cudaStreamDestroy(s);
         }
     } gr;
-    auto done = [&](int code) {
-        dev_free(c, d_c12, sizeof(float) * 2 * (size_t) nb);
-        return code;
-    };
     const MlpDev w = dev_of(m);
-    // the epochs' row orders in two page-locked buffers (the host shuffles
-    // the next epoch's while the device trains on the current one), and the
-    // epoch's bias corrections and losses in page-locked memory too, so that
-    // no copy of an epoch waits for the host or the host for the device
-    // before the shuffle is done
-    const size_t n = (size_t) m->n;
-    int *order[2] = {nullptr, nullptr};
-    float *c12 = nullptr, *losses = nullptr;
-    struct Pinned {
-        void *p[4];
-        ~Pinned()
-        {
-            for (void *q : p)
-                if (q) cudaFreeHost(q);
-        }
-    } pinned{};
     SplitMix rng{m->seed ^ 0x9e3779b97f4a7c15ull};
-    cudaError_t e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaHostAlloc(&pinned.p[0], sizeof(int) * n, 0);
-    if (e == cudaSuccess) e = cudaHostAlloc(&pinned.p[1], sizeof(int) * n, 0);
-    if (e == cudaSuccess) e = cudaHostAlloc(&pinned.p[2], sizeof(float) * 2 * (size_t) nb, 0);
-    if (e == cudaSuccess) e = cudaHostAlloc(&pinned.p[3], sizeof(float) * (size_t) nb, 0);
-    if (e != cudaSuccess) return done(cuda_fail(c, e, "training order buffers"));
-    order[0] = (int *) pinned.p[0];
-    order[1] = (int *) pinned.p[1];
-    c12 = (float *) pinned.p[2];
-    losses = (float *) pinned.p[3];
     for (size_t i = 0; i < n; i++) order[0][i] = (int) i;
     shuffle_rows(order[0], n, rng);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&gr.s, cudaStreamNonBlocking);
-    // the kernels' shared-memory attributes, set outside the capture
-    if (e == cudaSuccess) e = mlp_train_step(w, m->d_X, m->d_T, m->d_idx, 0, 1, wneg, IVR_MLP_TRANSPARENT, m->d_grad,
-                                             m->d_loss, gr.s);
-    // one epoch's mini-batches: gradient reset, training step, Adam (a
-    // launch-bound loop of 3 x nb launches, captured once)
-    if (e == cudaSuccess) e = cudaStreamBeginCapture(gr.s, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        cudaError_t ce = cudaSuccess;
-        for (long long b = 0; b < nb && ce == cudaSuccess; b++) {
+    e = cudaStreamCreateWithFlags(&gr.s, cudaStreamNonBlocking);
+    // one epoch's mini-batches: training step, Adam (which clears the gradient
+    // for the next step)
+    auto steps = [&]() {
+        cudaError_t se = cudaSuccess;
+        for (long long b = 0; b < nb && se == cudaSuccess; b++) {
             const long long r0 = b * batch_rows, rows = std::min<long long>(batch_rows, m->n - r0);
-            ce = cudaMemsetAsync(m->d_grad, 0, kParamBytes, gr.s);
-            if (ce == cudaSuccess)
-                ce = mlp_train_step(w, m->d_X, m->d_T, m->d_idx + r0, rows, rows, wneg, IVR_MLP_TRANSPARENT, m->d_grad,
-                                    m->d_loss + b, gr.s);
-            if (ce == cudaSuccess)
-                ce = mlp_adam(m->d_p, m->d_m, m->d_v, m->d_grad, lr, 0, d_c12 + 2 * b, m->d_w1t, m->d_w2t, m->d_w2,
+            se = mlp_train_step(w, m->d_X, m->d_T, m->d_idx + r0, rows, rows, wneg, IVR_MLP_TRANSPARENT, m->d_grad,
+                                m->d_loss + b, gr.s);
+            if (se == cudaSuccess)
+                se = mlp_adam(m->d_p, m->d_m, m->d_v, m->d_grad, lr, 0, d_c12 + 2 * b, m->d_w1t, m->d_w2t, m->d_w2,
                               gr.s);
         }
-        e = cudaStreamEndCapture(gr.s, &gr.g);
-        if (e == cudaSuccess) e = ce;
+        return se;
+    };
+    // A single epoch is launched as it is; several replay a captured one
+    // (2 x nb launches), so that the host is free to shuffle.
+    if (epochs > 1) {
+        // the kernels' shared-memory attributes, set outside the capture
+        if (e == cudaSuccess) e = mlp_train_step(w, m->d_X, m->d_T, m->d_idx, 0, 1, wneg, IVR_MLP_TRANSPARENT,
+                                                 m->d_grad, m->d_loss, gr.s);
+        if (e == cudaSuccess) e = cudaStreamBeginCapture(gr.s, cudaStreamCaptureModeThreadLocal);
+        if (e == cudaSuccess) {
+            const cudaError_t ce = steps();
+            e = cudaStreamEndCapture(gr.s, &gr.g);
+            if (e == cudaSuccess) e = ce;
+        }
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&gr.x, gr.g, 0);
     }
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&gr.x, gr.g, 0);
-    if (e != cudaSuccess) return done(cuda_fail(c, e, "training graph"));
+    if (e == cudaSuccess) e = cudaMemsetAsync(m->d_grad, 0, kParamBytes, gr.s);
+    if (e != cudaSuccess) return cuda_fail(c, e, "training graph");
     for (int ep = 0; ep < epochs; ep++) {
         const int cur = ep & 1;
         for (long long b = 0; b < nb; b++) mlp_adam_corrections(m->step + b + 1, &c12[2 * b], &c12[2 * b + 1]);
@@ -557,7 +560,7 @@ int ivr_mlp_train(ivr_mlp *m, int epochs, int batch_rows, float lr, float wneg, 
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d_c12, c12, sizeof(float) * 2 * (size_t) nb, cudaMemcpyHostToDevice, gr.s);
         if (e == cudaSuccess) e = cudaMemsetAsync(m->d_loss, 0, sizeof(float) * (size_t) nb, gr.s);
-        if (e == cudaSuccess) e = cudaGraphLaunch(gr.x, gr.s);
+        if (e == cudaSuccess) e = gr.x ? cudaGraphLaunch(gr.x, gr.s) : steps();
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(losses, m->d_loss, sizeof(float) * (size_t) nb, cudaMemcpyDeviceToHost, gr.s);
         if (e == cudaSuccess && ep + 1 < epochs) {  // the next epoch's order, meanwhile
@@ -565,7 +568,7 @@ int ivr_mlp_train(ivr_mlp *m, int epochs, int batch_rows, float lr, float wneg, 
             shuffle_rows(order[cur ^ 1], n, rng);
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(gr.s);  // c12 and the order buffers are rewritten next
-        if (e != cudaSuccess) return done(cuda_fail(c, e, "training epoch"));
+        if (e != cudaSuccess) return cuda_fail(c, e, "training epoch");
         m->step += (int) nb;
         if (loss_per_epoch) {
             double sum = 0.0;
@@ -576,12 +579,12 @@ int ivr_mlp_train(ivr_mlp *m, int epochs, int batch_rows, float lr, float wneg, 
     m->serial++;
     int status = 0;
     e = cudaMemcpy(&status, m->d_status, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return done(cuda_fail(c, e, "training status"));
+    if (e != cudaSuccess) return cuda_fail(c, e, "training status");
     if (status != 0) {
         cudaMemset(m->d_status, 0, sizeof(int));
-        return done(fail(c, IVR_ERR_TIMEOUT, "a tensor-core wait of the training step ran out; the parameters are suspect"));
+        return fail(c, IVR_ERR_TIMEOUT, "a tensor-core wait of the training step ran out; the parameters are suspect");
     }
-    return done(IVR_OK);
+    return IVR_OK;
 }
 
 int ivr_mlp_calibrate(ivr_mlp *m, float slack, float *margin, float *recall)

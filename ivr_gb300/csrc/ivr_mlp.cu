@@ -19,25 +19,37 @@ using bf16 = __nv_bfloat16;
 constexpr int F = kMlpIn;      // 32 (26 features, zero padded)
 constexpr int H = kMlpHidden;  // 64
 
-// Adam on the FP32 master parameters, then the BF16 operand copies
-// c12 (nullable): the bias corrections c1, c2 read from device memory
-// instead of the arguments (a launch that a CUDA graph replays every epoch)
-__global__ void mlp_adam_kernel(float *p, float *m, float *v, const float *gr, int np, float lr, float beta1,
-                                float beta2, float eps, float c1, float c2, const float *c12, bf16 *w1t, bf16 *w2t,
-                                bf16 *w2)
+// Adam on the FP32 master parameters, the BF16 operand copies of the ones
+// that have some, and the gradient cleared for the next step, in one launch
+// (launch-bound: with the copies and the clearing apart, a replayed step of
+// 1000 rows took 22.2 us, now 20.6).
+// c12 (nullable): the bias corrections c1, c2 read from device memory instead
+// of the arguments (a launch that a CUDA graph replays every epoch).
+__global__ void mlp_adam_kernel(float *p, float *m, float *v, float *gr, int np, float lr, float beta1, float beta2,
+                                float eps, float c1, float c2, const float *c12, bf16 *w1t, bf16 *w2t, bf16 *w2)
 {
     if (c12) {
         c1 = c12[0];
         c2 = c12[1];
     }
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-        float gi = gr[i];
-        if (i >= kOffW1 + kMlpFeatures * H && i < kOffW1 + F * H) gi = 0.0f;  // padding inputs
-        const float mi = beta1 * m[i] + (1.0f - beta1) * gi;
-        const float vi = beta2 * v[i] + (1.0f - beta2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= np) return;
+    float gi = gr[i];
+    gr[i] = 0.0f;
+    if (i >= kOffW1 + kMlpFeatures * H && i < kOffW1 + F * H) gi = 0.0f;  // padding inputs
+    const float mi = beta1 * m[i] + (1.0f - beta1) * gi;
+    const float vi = beta2 * v[i] + (1.0f - beta2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    const float q = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    p[i] = q;
+    if (i < kOffB1) {
+        const int f = i / H, u = i % H;  // W1[f][u]
+        w1t[u * F + f] = __float2bfloat16(q);
+    } else if (i >= kOffW2 && i < kOffB2) {
+        const int j = i - kOffW2, a = j / H, b = j % H;  // W2[a][b]
+        w2[j] = __float2bfloat16(q);
+        w2t[b * H + a] = __float2bfloat16(q);
     }
 }
 
@@ -184,15 +196,14 @@ void mlp_adam_corrections(long long step, float *c1, float *c2)
     *c2 = 1.0f - powf(0.999f, (float) step);
 }
 
-cudaError_t mlp_adam(float *p, float *m, float *v, const float *grad, float lr, int step, const float *c12,
-                     void *w1t, void *w2t, void *w2, cudaStream_t s)
+cudaError_t mlp_adam(float *p, float *m, float *v, float *grad, float lr, int step, const float *c12, void *w1t,
+                     void *w2t, void *w2, cudaStream_t s)
 {
     const float b1 = 0.9f, b2 = 0.999f;
     float c1 = 1.0f, c2 = 1.0f;
     if (!c12) mlp_adam_corrections(step, &c1, &c2);
-    mlp_adam_kernel<<<grid_of(kMlpParams, 256), 256, 0, s>>>(p, m, v, grad, kMlpParams, lr, b1, b2, 1e-8f, c1, c2,
-                                                             c12, (bf16 *) w1t, (bf16 *) w2t, (bf16 *) w2);
-    mlp_pack_kernel<<<grid_of(F * H + H * H, 256), 256, 0, s>>>(p, (bf16 *) w1t, (bf16 *) w2t, (bf16 *) w2);
+    mlp_adam_kernel<<<(kMlpParams + 63) / 64, 64, 0, s>>>(p, m, v, grad, kMlpParams, lr, b1, b2, 1e-8f, c1, c2, c12,
+                                                          (bf16 *) w1t, (bf16 *) w2t, (bf16 *) w2);
     return cudaGetLastError();
 }
 
