@@ -32,7 +32,8 @@ constexpr int kThreads = 128;
 // voxel pair) 512^3 at 1024x1024 392, 342, 357, 352 (395).  The batched
 // kernel reads its frames from global memory and has no tail: there more
 // warps win (f32, 32 frames: 3.84 ms at K = 2 with 8 blocks, 4.57 with 5,
-// 4.33 at K = 4 with 5).
+// 4.33 at K = 4 with 5; u16 and u8 1005 and 753 us at K = 2 with 8 blocks, 916
+// and 718 at K = 4 with 7).
 #ifndef IVR_K_INT
 #define IVR_K_INT 6
 #endif
@@ -42,16 +43,10 @@ constexpr int kThreads = 128;
 #ifndef IVR_CFG_BLOCKS_PER_SM
 #define IVR_CFG_BLOCKS_PER_SM 5
 #endif
-#ifndef IVR_K_BATCH
-#define IVR_K_BATCH 2
-#endif
-#ifndef IVR_BATCH_BLOCKS_PER_SM
-#define IVR_BATCH_BLOCKS_PER_SM 8
-#endif
 template <int DT> __host__ __device__ constexpr int cfg_k() { return DT == IVR_F32 ? IVR_K_F32 : IVR_K_INT; }
 constexpr int kCfgBlocksPerSm = IVR_CFG_BLOCKS_PER_SM;
-constexpr int kBatchK = IVR_K_BATCH;
-constexpr int kBatchBlocksPerSm = IVR_BATCH_BLOCKS_PER_SM;
+template <int DT> __host__ __device__ constexpr int batch_k() { return DT == IVR_F32 ? 2 : 4; }
+template <int DT> __host__ __device__ constexpr int batch_blocks_per_sm() { return DT == IVR_F32 ? 8 : 7; }
 constexpr int kPeakBlocksPerSm = 9;  // the sampler alone (sample_peak_kernel)
 
 template <int DT> struct VoxT;
@@ -1631,7 +1626,7 @@ cudaError_t launch_dt(const FrameDesc &f, float4 *o32, uchar4 *o8, cudaStream_t 
 // a binary search over the frames' first tiles.  Warp tiles are TW x (32/TW)
 // pixels; PAIR takes two samples per loop iteration.
 template <int DT, int TW, bool PAIR>
-__global__ void __launch_bounds__(kThreads, kBatchBlocksPerSm)
+__global__ void __launch_bounds__(kThreads, batch_blocks_per_sm<DT>())
     march_batch_kernel(const BatchHeader *__restrict__ hdr, const BatchItem *__restrict__ items,
                        unsigned long long *ticket)
 {
@@ -1654,7 +1649,7 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocksPerSm)
         }
         const BatchItem &it = items[lo];
         const long long tile = g - it.tile0;
-        pixel_cfg<DT, true, false, PAIR ? kBatchK : 1>(it.f, (int) (tile / it.tiles_x) * TH + lane / TW,
+        pixel_cfg<DT, true, false, PAIR ? batch_k<DT>() : 1>(it.f, (int) (tile / it.tiles_x) * TH + lane / TW,
                                         (int) (tile % it.tiles_x) * TW + lane % TW, it.out32, it.out8, nexec, nlat,
                                         s_runs + threadIdx.x);
     }
