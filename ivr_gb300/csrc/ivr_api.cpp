@@ -268,6 +268,7 @@ int tf_grid(ivr_volume *v, const ivr_tf *tf, bool zero_alpha, bool learned, cuda
     g->mlp_serial = mser;
     g->last_use = now;
     g->rejected = false;
+    g->after_build.clear();
     *(volatile int *) g->h_reject = 0;  // no launch that reads it is pending
     CK(c, cudaMemsetAsync(g->d_bad, 0, sizeof(int), s));
     // cell opacities (the tile order's input): an exact grid's only; learned
@@ -305,6 +306,32 @@ bool learned_rejected(ivr_volume::TfGrid *g)
 {
     if (!g->rejected) g->rejected = *(volatile int *) g->h_reject != 0;
     return g->rejected;
+}
+
+// Whether a plain CONFIG frame's launch on s may begin while the one before
+// it ends (launch_march's early).  All it reads before it waits for that launch
+// are the volume, the LUT and the grid, so the grid's build has to lie before
+// the launch it overlaps: the first launch on each stream after a build waits
+// for it, and those that follow may be early.  (Streams by their id: a handle
+// may be a new stream's.)  Not in a stream capture.
+int may_be_early(ivr_ctx *c, ivr_volume::TfGrid *grid, cudaStream_t s, bool *early)
+{
+    *early = false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(c, cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return IVR_OK;
+    if (grid) {
+        unsigned long long id = 0;
+        CK(c, cudaStreamGetId(s, &id));
+        auto &seen = grid->after_build;
+        if (std::find(seen.begin(), seen.end(), id) == seen.end()) {
+            CK(c, cudaStreamWaitEvent(s, grid->built, 0));
+            if (seen.size() < 64) seen.push_back(id);
+            return IVR_OK;
+        }
+    }
+    *early = true;
+    return IVR_OK;
 }
 
 // Fills everything of a launch's frame descriptor that depends on the TF,
@@ -385,7 +412,7 @@ int frame_for(ivr_view *view, ivr_tf *tf, int x, int y, int w, int h, int single
 }
 
 // One CONFIG/REF launch of f on the view's ticket counter.
-int launch_view(ivr_view *view, FrameDesc &f, float *o32, uint8_t *o8, cudaStream_t s)
+int launch_view(ivr_view *view, FrameDesc &f, float *o32, uint8_t *o8, cudaStream_t s, bool early)
 {
     ivr_ctx *c = view->ctx;
     if (view->tickets_dirty) {
@@ -396,7 +423,7 @@ int launch_view(ivr_view *view, FrameDesc &f, float *o32, uint8_t *o8, cudaStrea
     f.tickets = view->d_tickets;
     f.ticket_base = view->ticket_base;
     long long used = 0;
-    cudaError_t e = launch_march(f, (float4 *) o32, (uchar4 *) o8, s, &used);
+    cudaError_t e = launch_march(f, (float4 *) o32, (uchar4 *) o8, s, &used, early);
     if (e != cudaSuccess) {
         view->tickets_dirty = true;
         return cuda_fail(c, e, "march launch");
@@ -520,11 +547,16 @@ int render_window(ivr_view *view, ivr_tf *tf, int x, int y, int w, int h, int si
         f.judge8 = view->d_judge8;
     }
     int slot = -1;
-    if (!touched && grid && view->p.tile_order == IVR_TILES_COST) {
+    if (!touched && grid && view->p.tile_order == IVR_TILES_COST && tile_order_pays(f)) {
         rc = order_tiles(view, f, grid, exact, s, &slot);
         if (rc) return rc;
     }
-    rc = launch_view(view, f, o32, o8, s);
+    bool early = false;
+    if (f.preset == IVR_PRESET_CONFIG && !touched && !judged) {
+        rc = may_be_early(c, grid, s, &early);
+        if (rc) return rc;
+    }
+    rc = launch_view(view, f, o32, o8, s, early);
     if (rc == IVR_OK && judged) {
         const cudaError_t je = launch_judge_compare(f, (const uchar4 *) o8, (const float4 *) o32, s);
         if (je != cudaSuccess) rc = cuda_fail(c, je, "judge compare launch");
@@ -532,7 +564,7 @@ int render_window(ivr_view *view, ivr_tf *tf, int x, int y, int w, int h, int si
         ff.judge = nullptr;
         for (int k = 0; k < ff.nb; k++) ff.b[k].empty = exact->dist[k];
         ff.gate = &((JudgeWords *) view->d_judge)->fail;
-        if (rc == IVR_OK) rc = launch_view(view, ff, o32, o8, s);
+        if (rc == IVR_OK) rc = launch_view(view, ff, o32, o8, s, false);
     }
     if (slot >= 0) {  // the slot's readers, whether or not they launched
         CK(c, cudaEventRecord(view->tiles[slot].used, s));

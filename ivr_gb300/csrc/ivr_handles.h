@@ -55,6 +55,7 @@ struct ivr_volume {
         int *h_reject;
         int *d_reject;
         bool rejected;                // host has seen it: render with the exact grid
+        std::vector<unsigned long long> after_build;  // ids of the streams a launch of which has waited for `built`
     };
     std::vector<TfGrid *> grids;
     // learned skipping: the attached predictor, its margin, and per brick the

@@ -185,7 +185,10 @@ cudaError_t noalloc_histogram(const void *data, int dtype, long long n, int hsiz
 // march (ivr_march.cu)
 // *tickets: how many tile tickets the launch takes from f.tickets (a
 // persistent CONFIG launch takes each tile once and each warp fails once).
-cudaError_t launch_march(const FrameDesc &f, float4 *out32, uchar4 *out8, cudaStream_t s, long long *tickets);
+// early: the launch may begin before the one before it on s has ended
+// (nothing it reads is written there, and s is not being captured)
+cudaError_t launch_march(const FrameDesc &f, float4 *out32, uchar4 *out8, cudaStream_t s, long long *tickets,
+                         bool early);
 // the sampler alone on brick f.b[0] (sample-rate roofline): every thread
 // takes `steps` samples; *samples = threads * steps; out holds one float4 per
 // thread (sample_peak_threads())
@@ -203,6 +206,9 @@ cudaError_t launch_sample_peak(const FrameDesc &f, int layout, const SamplerTex 
 int sample_peak_threads();
 // the verdict of a learned-skip frame rendered by a judged launch of f
 cudaError_t launch_judge_compare(const FrameDesc &f, const uchar4 *out8, const float4 *out32, cudaStream_t s);
+// whether f has tiles enough for the estimated cost order to be worth its two
+// launches
+bool tile_order_pays(const FrameDesc &f);
 // bytes of f.judge8 a judged launch of f writes
 long long judge_scratch_bytes(const FrameDesc &f);
 // the CONFIG tile order of f, costliest first, into perm (ntiles ints) with
