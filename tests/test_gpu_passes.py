@@ -43,6 +43,24 @@ def test_minmax_and_histogram_match_the_oracle(ctx, oracle_mod, dtype, shape, to
         v.free()
 
 
+@pytest.mark.parametrize("dtype,n", [("u8", 70), ("u16", 140), ("f32", 80)])
+def test_histogram_of_plateaus(ctx, oracle_mod, dtype, n):
+    """Stretches of one value, longer and shorter than a 16-byte load and at
+    every offset in one: background, saturated and in between."""
+    rng = np.random.default_rng(11)
+    top = 255 if dtype != "u16" else 16383  # 140^3 voxels: shared counters, one copy
+    vals = rng.choice([0, 1, top // 3, top], 400000)
+    vol = np.repeat(vals, rng.integers(1, 41, vals.size))[:n ** 3]
+    vol = np.resize(vol, n ** 3).reshape(n, n, n).astype({"u8": np.uint8, "u16": np.uint16, "f32": np.float32}[dtype])
+    vol.reshape(-1)[:2] = (0, top)
+    _, _, ohist = oracle_mod.minmax_histogram(vol)
+    v = ctx.load_volume(vol)
+    try:
+        assert np.array_equal(v.histogram(len(ohist)), ohist)
+    finally:
+        v.free()
+
+
 def test_minmax_and_histogram_with_nan_and_infinite_voxels(ctx):
     """NaNs are no minimum or maximum and count as the bin (int)(NaN) = 0;
     an infinite voxel leaves every bin."""
