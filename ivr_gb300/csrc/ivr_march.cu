@@ -31,9 +31,9 @@ constexpr int kThreads = 128;
 // 200 (368); u8 128^3 at 256x256 69, 56, 51, 51 (80); f32 (four registers a
 // voxel pair) 512^3 at 1024x1024 392, 342, 357, 352 (395).  The batched
 // kernel reads its frames from global memory and has no tail: there more
-// warps win (f32, 32 frames: 3.84 ms at K = 2 with 8 blocks, 4.57 with 5,
-// 4.33 at K = 4 with 5; u16 and u8 1005 and 753 us at K = 2 with 8 blocks, 916
-// and 718 at K = 4 with 7).
+// warps win (32 f32 frames of a 512^3 volume: 3.67 ms at K = 2 with 8 blocks,
+// 3.74 with 9, 3.92 with 7; 20 u16 frames 2.53 ms at K = 4 with 8, 3.06 with
+// 7, 2.72 with 6, 2.88 at K = 2 with 9; u8 2.40, 2.37, 2.52, 2.59).
 #ifndef IVR_K_INT
 #define IVR_K_INT 6
 #endif
@@ -46,7 +46,7 @@ constexpr int kThreads = 128;
 template <int DT> __host__ __device__ constexpr int cfg_k() { return DT == IVR_F32 ? IVR_K_F32 : IVR_K_INT; }
 constexpr int kCfgBlocksPerSm = IVR_CFG_BLOCKS_PER_SM;
 template <int DT> __host__ __device__ constexpr int batch_k() { return DT == IVR_F32 ? 2 : 4; }
-template <int DT> __host__ __device__ constexpr int batch_blocks_per_sm() { return DT == IVR_F32 ? 8 : 7; }
+constexpr int kBatchBlocksPerSm = 8;
 constexpr int kPeakBlocksPerSm = 9;  // the sampler alone (sample_peak_kernel)
 
 template <int DT> struct VoxT;
@@ -365,19 +365,19 @@ struct CellPos {
 __device__ __forceinline__ CellPos cell_cfg(const DevBrick &b, float ux, float uy, float uz)
 {
     const int nx = b.nx, ny = b.ny, nz = b.nz;
-    // clamp to edge: the coordinate to [0, n-1], the cell to [0, n-2]; then
-    // the fraction u - floor(u) is exact and lies in [0, 1] (this gives the
-    // same cell and fraction as clamping the cell and then the fraction)
-    ux = fminf(fmaxf(ux, 0.0f), (float) (nx - 1));
-    uy = fminf(fmaxf(uy, 0.0f), (float) (ny - 1));
-    uz = fminf(fmaxf(uz, 0.0f), (float) (nz - 1));
+    // clamp to edge: the cell to [0, n-2] (the conversion takes what is
+    // negative to 0), the fraction to [0, 1] by the subtraction's saturation.
+    // u - floor(u) is exact, so this is the cell and the fraction of the
+    // coordinate clamped to [0, n-1] first, without the clamps' six
+    // instructions (f32 512^3 frame 347 -> 333 us, learned 1024^3 340 -> 328,
+    // u8 128^3 26.4 -> 25.0).  n is at least 2.
     CellPos c;
-    c.j = min(__float2int_rd(ux), nx - 2);
-    c.i = min(__float2int_rd(uy), ny - 2);
-    c.k = min(__float2int_rd(uz), nz - 2);
-    c.fx = ux - (float) c.j;
-    c.fy = uy - (float) c.i;
-    c.fz = uz - (float) c.k;
+    c.j = (int) min(__float2uint_rd(ux), (unsigned) (nx - 2));
+    c.i = (int) min(__float2uint_rd(uy), (unsigned) (ny - 2));
+    c.k = (int) min(__float2uint_rd(uz), (unsigned) (nz - 2));
+    c.fx = __saturatef(ux - (float) c.j);
+    c.fy = __saturatef(uy - (float) c.i);
+    c.fz = __saturatef(uz - (float) c.k);
     return c;
 }
 
@@ -907,6 +907,26 @@ constexpr int kRunMax = 8;
 constexpr unsigned kFullWarp = 0xffffffffu;
 static_assert(kRunSamples < 256, "run lengths have 8 bits");
 
+// A ray's direction, its reciprocals and the ray's lattice: in registers, or
+// (PARK) in the lane's column of a [kRayWords][kThreads] shared array, read
+// where they are used and out of the way while samples are taken.  The
+// batched kernel, which has 64 registers, parks: kept in registers they pushed
+// the sampling loop's own values into local memory, as many requests as all
+// its other loads (f32, 32 frames: 3.85 -> 3.76 ms, u16 20 frames 2.62 ->
+// 2.56).  The frame kernels have the registers and read what is uniform from
+// the constant bank.
+enum RayWord { kDx, kDy, kDz, kIdx, kIdy, kIdz, kT0, kDt, kIdt, kRayWords };
+template <bool PARK> struct Ray {
+    float v[kRayWords];
+    __device__ __forceinline__ void set(RayWord k, float x) { v[k] = x; }
+    __device__ __forceinline__ float operator[](RayWord k) const { return v[k]; }
+};
+template <> struct Ray<true> {
+    volatile float *v;
+    __device__ __forceinline__ void set(RayWord k, float x) { v[k * kThreads] = x; }
+    __device__ __forceinline__ float operator[](RayWord k) const { return v[k * kThreads]; }
+};
+
 // One brick of the CONFIG march with a skipping grid, in two alternating
 // steps.  (1) Each lane walks its ray over the macrocell grid and notes the
 // runs of lattice indices that lie in opaque cells, until it has
@@ -925,21 +945,22 @@ static_assert(kRunSamples < 256, "run lengths have 8 bits");
 // time).  Bound by the latency of the longest rays: of a 354 us f32 frame
 // (512^3, 1024x1024) the SMs have work for about 70%, with 43% of all issue
 // slots used.
-template <int DT, int K>
+template <int DT, int K, bool PARK>
 __device__ __forceinline__ void march_runs(const FrameDesc &f, const DevBrick &b, const uint8_t *empty,
-                                           unsigned *runs, bool in, float dx, float dy, float dz, float idx,
-                                           float idy, float idz, float t0, float dt, float idt, float4 &acc,
-                                           bool &done)
+                                           unsigned *runs, bool in, const Ray<PARK> &ray, float4 &acc, bool &done)
 {
+    const float dx = ray[kDx], dy = ray[kDy], dz = ray[kDz], idx = ray[kIdx], idy = ray[kIdy], idz = ray[kIdz];
+    const float t0 = ray[kT0], dt = ray[kDt], idt = ray[kIdt];
     float tin, tout;
     in = in && ray_box_cfg(b.dconst, f.origx, f.origy, f.origz, dx, dy, dz, idx, idy, idz, tin, tout);
     int i = in ? cfg_first_ge(t0, dt, idt, tin) : 0;  // the next lattice index to look at
     int i1 = in ? cfg_first_ge(t0, dt, idt, tout) : 0;
     const float opac = f.alpha, term = f.term_alpha;
     const VoxLattice L = vox_lattice(b, f.origx, f.origy, f.origz, dx, dy, dz, t0, dt);
-    const float isx = idx * idt * b.vwx, isy = idy * idt * b.vwy, isz = idz * idt * b.vwz;
     int held = i;  // indices i..held-1 lie in an opaque cell already checked
     while (__any_sync(kFullWarp, i < i1)) {
+        const float isx = ray[kIdx] * ray[kIdt] * b.vwx, isy = ray[kIdy] * ray[kIdt] * b.vwy,
+                    isz = ray[kIdz] * ray[kIdt] * b.vwz;
         int nr = 0, n = 0;       // runs noted, samples in them
         int start = 0, len = 0;  // the run being built
         bool walk = i < i1;
@@ -1084,9 +1105,10 @@ __global__ void __launch_bounds__(kThreads, kRefBlocksPerSm) march_ref_kernel(co
 // One CONFIG ray per lane: pixel (i, j) of the viewport, all bricks front to
 // back, skipping by the bricks' grids, or by the exact grids f.exact when
 // exact.  Every lane of the warp calls it; one with `live` false has no ray.
-template <int DT, bool SKIP, bool CENSUS, int K>
+template <int DT, bool SKIP, bool CENSUS, int K, bool PARK = false>
 __device__ __forceinline__ float4 ray_cfg(const FrameDesc &f, int i, int j, bool live, unsigned long long &nexec,
-                                          unsigned long long &nlat, unsigned *runs, bool exact = false)
+                                          unsigned long long &nlat, unsigned *runs, bool exact = false,
+                                          volatile float *park = nullptr)
 {
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     bool any = false;
@@ -1107,6 +1129,17 @@ __device__ __forceinline__ float4 ray_cfg(const FrameDesc &f, int i, int j, bool
     const float dt = f.step / len;
     bool done = !live || !(dt > 0.0f);
     const float idt = 1.0f / dt;
+    Ray<PARK> ray;
+    if constexpr (PARK) ray.v = park;
+    ray.set(kDx, dx);
+    ray.set(kDy, dy);
+    ray.set(kDz, dz);
+    ray.set(kIdx, idx);
+    ray.set(kIdy, idy);
+    ray.set(kIdz, idz);
+    ray.set(kT0, t0);
+    ray.set(kDt, dt);
+    ray.set(kIdt, idt);
     for (int s = 0; s < f.nb; s++) {
         const int k = f.order[s];
         if (f.single >= 0 && k != f.single) continue;
@@ -1120,22 +1153,25 @@ __device__ __forceinline__ float4 ray_cfg(const FrameDesc &f, int i, int j, bool
             else if (in)
                 march_census<DT, false>(f, b, empty, dx, dy, dz, idx, idy, idz, t0, dt, idt, acc, done, nexec, nlat);
         } else if (SKIP && empty != nullptr) {
-            march_runs<DT, K>(f, b, empty, runs, in, dx, dy, dz, idx, idy, idz, t0, dt, idt, acc, done);
+            march_runs<DT, K, PARK>(f, b, empty, runs, in, ray, acc, done);
         } else if (in) {
-            march_plain<DT, K>(f, b, dx, dy, dz, idx, idy, idz, t0, dt, idt, acc, done);
+            march_plain<DT, K>(f, b, ray[kDx], ray[kDy], ray[kDz], ray[kIdx], ray[kIdy], ray[kIdz], ray[kT0], ray[kDt],
+                               ray[kIdt], acc, done);
         }
     }
     return acc;
 }
 
 // One pixel of the output window (ow, oh) = (oj, oi).
-template <int DT, bool SKIP, bool CENSUS, int K>
+template <int DT, bool SKIP, bool CENSUS, int K, bool PARK>
 __device__ __forceinline__ float4 pixel_cfg(const FrameDesc &f, int oi, int oj, float4 *out32, uchar4 *out8,
-                                            unsigned long long &nexec, unsigned long long &nlat, unsigned *runs)
+                                            unsigned long long &nexec, unsigned long long &nlat, unsigned *runs,
+                                            volatile float *park)
 {
     const bool in_window = oj < f.out_w && oi < f.out_h;
     const int j = f.out_x + oj, i = f.out_y + oi;
-    const float4 acc = ray_cfg<DT, SKIP, CENSUS, K>(f, i, j, in_window && i < f.vh && j < f.vw, nexec, nlat, runs);
+    const float4 acc = ray_cfg<DT, SKIP, CENSUS, K, PARK>(f, i, j, in_window && i < f.vh && j < f.vw, nexec, nlat,
+                                                          runs, false, park);
     if (!in_window) return acc;
     const long long o = (long long) oi * f.out_w + oj;
     if (out32) out32[o] = acc;
@@ -1656,12 +1692,13 @@ cudaError_t launch_dt(const FrameDesc &f, float4 *o32, uchar4 *o8, cudaStream_t 
 // a binary search over the frames' first tiles.  Warp tiles are TW x (32/TW)
 // pixels; PAIR takes two samples per loop iteration.
 template <int DT, int TW, bool PAIR>
-__global__ void __launch_bounds__(kThreads, batch_blocks_per_sm<DT>())
+__global__ void __launch_bounds__(kThreads, kBatchBlocksPerSm)
     march_batch_kernel(const BatchHeader *__restrict__ hdr, const BatchItem *__restrict__ items,
                        unsigned long long *ticket)
 {
     constexpr int TH = 32 / TW;
     __shared__ unsigned s_runs[kRunMax * kThreads];
+    __shared__ float s_ray[kRayWords * kThreads];
     const int lane = threadIdx.x & 31;
     const int n = hdr->nitems;
     const long long total = hdr->total_tiles;
@@ -1679,9 +1716,9 @@ __global__ void __launch_bounds__(kThreads, batch_blocks_per_sm<DT>())
         }
         const BatchItem &it = items[lo];
         const long long tile = g - it.tile0;
-        pixel_cfg<DT, true, false, PAIR ? batch_k<DT>() : 1>(it.f, (int) (tile / it.tiles_x) * TH + lane / TW,
+        pixel_cfg<DT, true, false, PAIR ? batch_k<DT>() : 1, true>(it.f, (int) (tile / it.tiles_x) * TH + lane / TW,
                                         (int) (tile % it.tiles_x) * TW + lane % TW, it.out32, it.out8, nexec, nlat,
-                                        s_runs + threadIdx.x);
+                                        s_runs + threadIdx.x, s_ray + threadIdx.x);
     }
 }
 
