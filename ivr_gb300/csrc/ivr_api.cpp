@@ -81,16 +81,107 @@ namespace {
 
 using namespace ivr;
 
+// An array of a block: *p its address, null until it is allocated.
+struct BlockArray {
+    void **p;
+    size_t bytes;
+    bool optional;  // left out where there is no room for it
+};
+
+// The driver takes some 30 us to allocate an array, 30 to free one, and 0.3 and
+// 0.5 us a megabyte more.  Eight bricks have 24 arrays, their skipping grid 17:
+// arrays that live and die together are parts of one block (384^3 f32 volume,
+// 2x2x2 bricks, opened up to its first frame: 5.2 -> 4.8 ms, and 3.8 with the
+// corner-packed copies' block kept from layout to layout).
+constexpr size_t kBlockAlign = 512;
+
+size_t block_bytes(const std::vector<BlockArray> &arrays)
+{
+    size_t n = 0;
+    for (const auto &a : arrays) n += (a.bytes + kBlockAlign - 1) / kBlockAlign * kBlockAlign;
+    return n;
+}
+
+void place(const std::vector<BlockArray> &arrays, void *block)
+{
+    char *p = (char *) block;
+    for (const auto &a : arrays) {
+        if (a.bytes) *a.p = p;
+        p += (a.bytes + kBlockAlign - 1) / kBlockAlign * kBlockAlign;
+    }
+}
+
+// Each array by itself, where the device has no block for all of them.
+int alloc_each(ivr_ctx *c, const std::vector<BlockArray> &arrays)
+{
+    for (const auto &a : arrays) {
+        const std::string err = c->err;
+        const int rc = dev_alloc(c, a.bytes, a.p);
+        if (rc && !a.optional) return rc;
+        if (rc) c->err = err;
+    }
+    return IVR_OK;
+}
+
+// What the budget admits of the arrays, one after the other: the others get 0
+// bytes, *used what the context then uses.
+int admit(ivr_ctx *c, std::vector<BlockArray> &arrays, size_t *used)
+{
+    *used = c->used;
+    for (auto &a : arrays) {
+        if (c->budget && a.bytes && *used + a.bytes > c->budget) {
+            if (!a.optional)
+                return fail(c, IVR_ERR_NOMEM, "HBM budget: %zu + %zu bytes exceeds %zu", *used, a.bytes, c->budget);
+            a.bytes = 0;
+        }
+        *used += a.bytes;
+    }
+    return IVR_OK;
+}
+
+// *block null afterwards: each array has an allocation of its own.
+int alloc_block(ivr_ctx *c, std::vector<BlockArray> arrays, void **block)
+{
+    size_t used = 0;
+    *block = nullptr;
+    const int rc = admit(c, arrays, &used);
+    if (rc) return rc;
+    if (cudaMalloc(block, block_bytes(arrays)) != cudaSuccess) {
+        cudaGetLastError();
+        *block = nullptr;
+        return alloc_each(c, arrays);
+    }
+    place(arrays, *block);
+    c->used = used;
+    return IVR_OK;
+}
+
+void free_block(ivr_ctx *c, const std::vector<BlockArray> &arrays, void *block)
+{
+    for (const auto &a : arrays) {
+        if (!block) dev_free(c, *a.p, a.bytes);
+        else if (*a.p) c->used -= a.bytes;
+        *a.p = nullptr;
+    }
+    cudaFree(block);
+}
+
+std::vector<BlockArray> grid_arrays(const ivr_volume *v, ivr_volume::TfGrid *g)
+{
+    std::vector<BlockArray> a = {{(void **) &g->d_bad, sizeof(int), false}};
+    for (size_t k = 0; k < g->dist.size(); k++) {
+        a.push_back({(void **) &g->dist[k], mc_cells(v->bricks[k]), false});
+        a.push_back({(void **) &g->opac[k], mc_cells(v->bricks[k]), false});
+    }
+    return a;
+}
+
 void delete_grid(ivr_volume *v, ivr_volume::TfGrid *g)
 {
-    for (size_t k = 0; k < g->dist.size(); k++)
-        if (g->dist[k]) dev_free(v->ctx, g->dist[k], mc_cells(v->bricks[k]));
-    for (size_t k = 0; k < g->opac.size(); k++)
-        if (g->opac[k]) dev_free(v->ctx, g->opac[k], mc_cells(v->bricks[k]));
+    free_block(v->ctx, grid_arrays(v, g), g->block);
     if (g->ev) cudaEventDestroy(g->ev);
     if (g->built) cudaEventDestroy(g->built);
     if (g->h_reject) cudaFreeHost(g->h_reject);
-    if (g->d_bad) dev_free(v->ctx, g->d_bad, sizeof(int));
     delete g;
 }
 
@@ -116,30 +207,89 @@ void free_grids(ivr_volume *v)
     v->grids.clear();
 }
 
-void free_bricks(ivr_volume *v)
+// Voxels (where the brick is not the volume), macrocells and the corner-packed
+// copy of each brick, in the order in which the budget admits them.  The copy is
+// an accelerator: without room for it the march reads the brick itself.
+std::vector<BlockArray> brick_arrays(ivr_volume *v)
+{
+    std::vector<BlockArray> a;
+    for (auto &b : v->bricks) {
+        if (b.owns) a.push_back({&b.data, brick_bytes(v, b), false});
+        a.push_back({(void **) &b.mc_minmax, mc_cells(b) * 2 * sizeof(float), false});
+        a.push_back({&b.quad, v->quads ? quad_bytes(v->dtype, b.lw, b.lh, b.ld) : 0, true});
+    }
+    return a;
+}
+
+void free_quad_block(ivr_volume *v)
+{
+    cudaFree(v->quad_block);
+    v->quad_block = nullptr;
+    v->quad_cap = 0;
+}
+
+// keep_quads: the copies' block stays for the layout that follows.
+void free_bricks(ivr_volume *v, bool keep_quads = false)
 {
     free_grids(v);
     learned_release(v);
     for (auto &b : v->bricks) {
-        if (b.owns) dev_free(v->ctx, b.data, brick_bytes(v, b));
-        dev_free(v->ctx, b.mc_minmax, mc_cells(b) * 2 * sizeof(float));
-        if (b.quad) dev_free(v->ctx, b.quad, quad_bytes(v->dtype, b.lw, b.lh, b.ld));
+        const BlockArray own[2] = {{&b.data, b.owns ? brick_bytes(v, b) : 0, false},
+                                   {(void **) &b.mc_minmax, mc_cells(b) * 2 * sizeof(float), false}};
+        for (const auto &a : own) {
+            if (a.bytes == 0 || !*a.p) continue;
+            if (v->brick_block) v->ctx->used -= a.bytes;
+            else dev_free(v->ctx, *a.p, a.bytes);
+        }
+        if (!b.quad) continue;
+        const size_t qb = quad_bytes(v->dtype, b.lw, b.lh, b.ld);
+        if (v->quad_block) v->ctx->used -= qb;
+        else dev_free(v->ctx, b.quad, qb);
     }
+    cudaFree(v->brick_block);
+    v->brick_block = nullptr;
+    if (!keep_quads) free_quad_block(v);
     v->bricks.clear();
 }
 
-// macrocell grid over a brick's local voxels (cells of the volume's edge,
-// +1 layer)
-int build_macrocells(ivr_volume *v, HostBrick &b)
+// The bricks' arrays in two blocks, the corner-packed copies' of its own: they
+// are four times the volume and nearly the same size in every layout, so the
+// block of one layout (that of the whole volume, which every volume starts
+// with) serves the next.  It has kQuadSpare slabs to spare for the halos.
+// Under a budget it is neither kept nor larger than what was admitted.
+constexpr int kQuadSpare = 3;
+int alloc_bricks(ivr_volume *v)
 {
-    b.cell = v->cell;
-    b.mcx = (b.lw - 2) / b.cell + 1;
-    b.mcy = (b.lh - 2) / b.cell + 1;
-    b.mcz = (b.ld - 2) / b.cell + 1;
-    int rc = dev_alloc(v->ctx, mc_cells(b) * 2 * sizeof(float), (void **) &b.mc_minmax);
+    ivr_ctx *c = v->ctx;
+    std::vector<BlockArray> arrays = brick_arrays(v), must, quads;
+    size_t used = 0;
+    int rc = admit(c, arrays, &used);
     if (rc) return rc;
-    CK(v->ctx, launch_macrocells(b.data, v->dtype, b.lw, b.lh, b.ld, b.cell, b.mc_minmax, b.mcx, b.mcy, b.mcz, 0));
-    return IVR_OK;
+    for (const auto &a : arrays) (a.optional ? quads : must).push_back(a);
+    const size_t need = block_bytes(must), qneed = block_bytes(quads);
+    if (qneed > v->quad_cap || qneed == 0) free_quad_block(v);
+    cudaError_t e = cudaMalloc(&v->brick_block, need);
+    if (e != cudaSuccess && v->quad_block) {
+        free_quad_block(v);
+        e = cudaMalloc(&v->brick_block, need);
+    }
+    if (e != cudaSuccess) v->brick_block = nullptr;
+    if (e == cudaSuccess && qneed && !v->quad_block) {
+        const size_t spare = c->budget ? 0 : kQuadSpare * quad_bytes(v->dtype, v->w, v->h, 1);
+        e = cudaMalloc(&v->quad_block, qneed + spare);
+        if (e == cudaSuccess) v->quad_cap = qneed + spare;
+        else v->quad_block = nullptr;
+    }
+    if (e == cudaSuccess) {
+        place(must, v->brick_block);
+        if (qneed) place(quads, v->quad_block);
+        c->used = used;
+        return IVR_OK;
+    }
+    cudaGetLastError();
+    cudaFree(v->brick_block);
+    v->brick_block = nullptr;
+    return alloc_each(c, arrays);
 }
 
 int setup_bricks(ivr_volume *v, int py, int px, int pz, int overlap)
@@ -149,7 +299,8 @@ int setup_bricks(ivr_volume *v, int py, int px, int pz, int overlap)
         return fail(c, IVR_ERR_INVALID, "brick grid %dx%dx%d (overlap %d) not supported", py, px, pz, overlap);
     if (v->w / px < 2 || v->h / py < 2 || v->d / pz < 2)
         return fail(c, IVR_ERR_INVALID, "bricks of %dx%dx%d voxels are too thin", v->w / px, v->h / py, v->d / pz);
-    free_bricks(v);
+    CK(c, cudaDeviceSynchronize());  // frames in flight read the copies whose block is kept
+    free_bricks(v, v->quads && !c->budget);
     v->layout++;
     int K = py * px * pz;
     v->bricks.resize(K);
@@ -157,28 +308,22 @@ int setup_bricks(ivr_volume *v, int py, int px, int pz, int overlap)
         HostBrick &b = v->bricks[r];
         memset(&b, 0, sizeof(b));
         brick_geometry(v->w, v->h, v->d, py, px, pz, overlap, r, b);
-        if (K == 1) {
-            b.data = v->d_full;
-            b.owns = false;
-        } else {
-            int rc = dev_alloc(c, brick_bytes(v, b), &b.data);
-            if (rc) { free_bricks(v); return rc; }
-            b.owns = true;
+        b.owns = K > 1;
+        if (K == 1) b.data = v->d_full;
+        // macrocells over the brick's local voxels, halo included
+        b.cell = v->cell;
+        b.mcx = (b.lw - 2) / b.cell + 1;
+        b.mcy = (b.lh - 2) / b.cell + 1;
+        b.mcz = (b.ld - 2) / b.cell + 1;
+    }
+    const int rc = alloc_bricks(v);
+    if (rc) { free_bricks(v); return rc; }
+    for (auto &b : v->bricks) {
+        if (b.owns)
             CK(c, launch_gather_brick(v->d_full, v->w, v->h, v->d, b.data, b.sx, b.sy, b.sz, b.lw, b.lh, b.ld,
                                       (int) dtype_size(v->dtype), 0));
-        }
-        int rc = build_macrocells(v, b);
-        if (rc) { free_bricks(v); return rc; }
-        if (v->quads) {
-            // the corner-packed copy is an accelerator: without room for it
-            // the march reads the brick itself
-            const size_t qb = quad_bytes(v->dtype, b.lw, b.lh, b.ld);
-            const std::string err = c->err;
-            if (dev_alloc(c, qb, &b.quad) == IVR_OK)
-                CK(c, launch_quads(b.data, v->dtype, b.lw, b.lh, b.ld, b.quad, 0));
-            else
-                c->err = err;
-        }
+        CK(c, launch_macrocells(b.data, v->dtype, b.lw, b.lh, b.ld, b.cell, b.mc_minmax, b.mcx, b.mcy, b.mcz, 0));
+        if (b.quad) CK(c, launch_quads(b.data, v->dtype, b.lw, b.lh, b.ld, b.quad, 0));
     }
     CK(c, cudaDeviceSynchronize());
     v->py = py; v->px = px; v->pz = pz; v->overlap = overlap;
@@ -237,25 +382,32 @@ int tf_grid(ivr_volume *v, const ivr_tf *tf, bool zero_alpha, bool learned, cuda
     if (v->grids.size() >= kMaxTfGrids)
         for (auto *h : v->grids)
             if (h->last_use < protect_from && (!g || h->last_use < g->last_use)) g = h;
+    // the judge's verdict word: a learned grid's only (the driver takes 250 us
+    // to allocate and free one)
+    auto has_verdict = [&](ivr_volume::TfGrid *q) {
+        if (!learned || q->h_reject) return true;
+        if (cudaHostAlloc((void **) &q->h_reject, sizeof(int), cudaHostAllocMapped) == cudaSuccess &&
+            cudaHostGetDevicePointer((void **) &q->d_reject, q->h_reject, 0) == cudaSuccess)
+            return true;
+        cudaGetLastError();
+        if (q->h_reject) cudaFreeHost(q->h_reject);
+        q->h_reject = nullptr;
+        return false;
+    };
     if (g) {
         CK(c, cudaEventSynchronize(g->ev));
+        if (!has_verdict(g)) return fail(c, IVR_ERR_CUDA, "events for a distance field");
     } else {
         g = new ivr_volume::TfGrid();
         g->dist.assign(v->bricks.size(), nullptr);
         g->opac.assign(v->bricks.size(), nullptr);
         int rc = IVR_OK;
         if (cudaEventCreateWithFlags(&g->ev, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&g->built, cudaEventDisableTiming) != cudaSuccess ||
-            cudaHostAlloc((void **) &g->h_reject, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-            cudaHostGetDevicePointer((void **) &g->d_reject, g->h_reject, 0) != cudaSuccess) {
+            cudaEventCreateWithFlags(&g->built, cudaEventDisableTiming) != cudaSuccess || !has_verdict(g)) {
             cudaGetLastError();
             rc = IVR_ERR_CUDA;
         }
-        if (rc == IVR_OK) rc = dev_alloc(c, sizeof(int), (void **) &g->d_bad);
-        for (size_t k = 0; k < v->bricks.size() && rc == IVR_OK; k++) {
-            rc = dev_alloc(c, mc_cells(v->bricks[k]), (void **) &g->dist[k]);
-            if (rc == IVR_OK) rc = dev_alloc(c, mc_cells(v->bricks[k]), (void **) &g->opac[k]);
-        }
+        if (rc == IVR_OK) rc = alloc_block(c, grid_arrays(v, g), &g->block);
         if (rc) {
             delete_grid(v, g);
             return rc == IVR_ERR_CUDA ? fail(c, rc, "events for a distance field") : rc;
@@ -269,7 +421,7 @@ int tf_grid(ivr_volume *v, const ivr_tf *tf, bool zero_alpha, bool learned, cuda
     g->last_use = now;
     g->rejected = false;
     g->after_build.clear();
-    *(volatile int *) g->h_reject = 0;  // no launch that reads it is pending
+    if (g->h_reject) *(volatile int *) g->h_reject = 0;  // no launch that reads it is pending
     CK(c, cudaMemsetAsync(g->d_bad, 0, sizeof(int), s));
     // cell opacities (the tile order's input): an exact grid's only; learned
     // frames use those of their TF's exact grid

@@ -28,6 +28,9 @@ struct ivr_volume {
     void *d_full = nullptr;
     size_t full_bytes = 0;
     std::vector<ivr::HostBrick> bricks;
+    void *brick_block = nullptr;  // holds the bricks' voxels and macrocells (null: one allocation each)
+    void *quad_block = nullptr;   // holds their corner-packed copies (null: one allocation each)
+    size_t quad_cap = 0;          // its bytes
     int py = 1, px = 1, pz = 1, overlap = 0;
     bool quads = true;  // keep corner-packed copies of the bricks (HostBrick::quad)
     int cell = ivr::kCell;  // macrocell edge in voxels (ivr_volume_set_macrocell)
@@ -43,6 +46,7 @@ struct ivr_volume {
         int learned;
         unsigned mlp_serial;          // learned: the predictor's parameter version
         unsigned long long last_use;  // ctx grid_clock
+        void *block;                  // holds d_bad, dist and opac (null: one allocation each)
         std::vector<uint8_t *> dist;  // per brick
         std::vector<uint8_t *> opac;  // per brick: DevBrick::opac (the exact rule's)
         cudaEvent_t ev;               // after the last launch that read it
