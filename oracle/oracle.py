@@ -66,7 +66,7 @@ def build(ref: bool | None = None) -> None:
     """make the oracles: O2 always, O1 when the reference sources exist."""
     subprocess.run(["make", "-s", "-C", HERE, "oracle"], check=True)
     if ref is None:
-        ref = os.path.isdir(REF_SRC)
+        ref = os.path.exists(os.path.join(REF_SRC, "ray.c"))  # an empty checkout is none
     if ref:
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF={REF_SRC}"], check=True)
 
