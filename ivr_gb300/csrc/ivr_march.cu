@@ -45,6 +45,13 @@ constexpr int kThreads = 128;
 #endif
 template <int DT> __host__ __device__ constexpr int cfg_k() { return DT == IVR_F32 ? IVR_K_F32 : IVR_K_INT; }
 constexpr int kCfgBlocksPerSm = IVR_CFG_BLOCKS_PER_SM;
+// Launches without any grid take their samples in packed pairs, six at a time
+// for every type (us a frame of a 301x260x223 volume, 4, 6, 8 samples: u16
+// 853x479 202, 182, 194 against 186 unpacked; f32 1024x1024 560, 535, 553
+// against 572; u8 1024x1024 472 against 497).  With a grid, packing loses: its
+// pairs cost the run loop registers (u16 learned 341 -> 383, the batched
+// kernel 3.85 -> 3.91 ms).
+constexpr int kPlainK = 6;
 template <int DT> __host__ __device__ constexpr int batch_k() { return DT == IVR_F32 ? 2 : 4; }
 constexpr int kBatchBlocksPerSm = 8;
 constexpr int kPeakBlocksPerSm = 9;  // the sampler alone (sample_peak_kernel)
@@ -522,6 +529,45 @@ __device__ __forceinline__ float quad_interp(const QuadCell<DT> &q, const CellPo
     return lerpf(c0, c1, c.fz);
 }
 
+// Two samples' interpolation in packed FP32 instructions, each lane rounding
+// as the scalar code above does: b - a is one fma by -1 (an exact product), so
+// no product feeds a sum.
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, f2(-1.0f), a); }
+__device__ __forceinline__ F2 f2_lerp(F2 a, F2 b, F2 t) { return f2_fma(t, f2_sub(b, a), a); }
+__device__ __forceinline__ F2 f2_lerp23(F2 A, F2 B, F2 t) { return f2_fma(t, f2_sub(B, A), A + f2(-8388608.0f)); }
+
+// quad_interp of two loaded cells
+template <int DT>
+__device__ __forceinline__ void quad_interp2(const QuadCell<DT> &p, const QuadCell<DT> &q, const CellPos &c,
+                                             const CellPos &d, float &s0, float &s1)
+{
+    const F2 fx = f2(c.fx, d.fx), fy = f2(c.fy, d.fy), fz = f2(c.fz, d.fz);
+    F2 c00, c10, c01, c11;
+    if constexpr (DT == IVR_U8) {
+        auto v = [](unsigned a, unsigned b, unsigned lane) { return f2(off23(a, lane), off23(b, lane)); };
+        c00 = f2_lerp23(v(p.lo, q.lo, kU8Lane0), v(p.lo, q.lo, kU8Lane1), fx);
+        c10 = f2_lerp23(v(p.lo, q.lo, kU8Lane2), v(p.lo, q.lo, kU8Lane3), fx);
+        c01 = f2_lerp23(v(p.hi, q.hi, kU8Lane0), v(p.hi, q.hi, kU8Lane1), fx);
+        c11 = f2_lerp23(v(p.hi, q.hi, kU8Lane2), v(p.hi, q.hi, kU8Lane3), fx);
+    } else if constexpr (DT == IVR_U16) {
+        auto v = [](unsigned a, unsigned b, unsigned half) { return f2(off23(a, half), off23(b, half)); };
+        c00 = f2_lerp23(v(p.lo.x, q.lo.x, kU16Half0), v(p.lo.x, q.lo.x, kU16Half1), fx);
+        c10 = f2_lerp23(v(p.lo.y, q.lo.y, kU16Half0), v(p.lo.y, q.lo.y, kU16Half1), fx);
+        c01 = f2_lerp23(v(p.hi.x, q.hi.x, kU16Half0), v(p.hi.x, q.hi.x, kU16Half1), fx);
+        c11 = f2_lerp23(v(p.hi.y, q.hi.y, kU16Half0), v(p.hi.y, q.hi.y, kU16Half1), fx);
+    } else {
+        auto x = [&](float a0, float b0, float a1, float b1) {
+            return kQuadDelta ? f2(fmaf(c.fx, b0, a0), fmaf(d.fx, b1, a1))
+                              : f2(lerpf(a0, b0, c.fx), lerpf(a1, b1, d.fx));
+        };
+        c00 = x(p.lo.x, p.lo.y, q.lo.x, q.lo.y);
+        c10 = x(p.lo.z, p.lo.w, q.lo.z, q.lo.w);
+        c01 = x(p.hi.x, p.hi.y, q.hi.x, q.hi.y);
+        c11 = x(p.hi.z, p.hi.w, q.hi.z, q.hi.w);
+    }
+    f2_split(f2_lerp(f2_lerp(c00, c10, fy), f2_lerp(c01, c11, fy), fz), s0, s1);
+}
+
 // A ray's CONFIG lattice in a brick's voxel coordinates: lattice index i
 // samples u_i = fmaf(i, s, base) per axis, with s = (d * ic) * dt and
 // base = fmaf(d * ic, t0, (o - bmin) * ic) -- the point o + t_i d, t_i =
@@ -743,15 +789,28 @@ __device__ __forceinline__ int cfg_first_ge(float t0, float dt, float idt, float
 
 // K consecutive samples of a ray from lattice index fi: every load is issued
 // before the first interpolation.  Samples past the ray's run are harmless:
-// cell_cfg clamps the cells.
-template <int DT, int K>
+// cell_cfg clamps the cells.  PACK: in packed pairs (K even).
+template <int DT, int K, bool PACK>
 __device__ __forceinline__ void sample_run(const DevBrick &b, const VoxLattice &L, float fi, float (&s)[K])
 {
     CellPos c[K];
+    if constexpr (PACK) {
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-        const float fk = fi + (float) k;  // (float) (i + k): i < 2^24
-        c[k] = cell_cfg(b, fmaf(fk, L.sx, L.bx), fmaf(fk, L.sy, L.by), fmaf(fk, L.sz, L.bz));
+        for (int k = 0; k < K; k += 2) {
+            const F2 fk = f2(fi + (float) k, fi + (float) (k + 1));
+            float ux[2], uy[2], uz[2];
+            f2_split(f2_fma(fk, f2(L.sx), f2(L.bx)), ux[0], ux[1]);
+            f2_split(f2_fma(fk, f2(L.sy), f2(L.by)), uy[0], uy[1]);
+            f2_split(f2_fma(fk, f2(L.sz), f2(L.bz)), uz[0], uz[1]);
+            c[k] = cell_cfg(b, ux[0], uy[0], uz[0]);
+            c[k + 1] = cell_cfg(b, ux[1], uy[1], uz[1]);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const float fk = fi + (float) k;  // (float) (i + k): i < 2^24
+            c[k] = cell_cfg(b, fmaf(fk, L.sx, L.bx), fmaf(fk, L.sy, L.by), fmaf(fk, L.sz, L.bz));
+        }
     }
     if (b.quad) {
         // Every sample loads its own cell, also where two share one: a copy
@@ -762,7 +821,10 @@ __device__ __forceinline__ void sample_run(const DevBrick &b, const VoxLattice &
 #pragma unroll
         for (int k = 0; k < K; k++) q[k] = quad_load<DT>(b, quad_key(b, c[k]));
 #pragma unroll
-        for (int k = 0; k < K; k++) s[k] = quad_interp<DT>(q[k], c[k]);
+        for (int k = 0; k < K; k += PACK ? 2 : 1) {
+            if constexpr (PACK) quad_interp2<DT>(q[k], q[k + 1], c[k], c[k + 1], s[k], s[k + 1]);
+            else s[k] = quad_interp<DT>(q[k], c[k]);
+        }
     } else {
 #pragma unroll
         for (int k = 0; k < K; k++) s[k] = fetch_cfg<DT>(b, c[k]);
@@ -842,7 +904,7 @@ __device__ __forceinline__ bool look_cell(const DevBrick &b, const uint8_t *empt
 
 // One brick of the CONFIG march without skipping: samples tin_k <= t_i <
 // tout_k of the ray's lattice, front-to-back into acc, K per iteration.
-template <int DT, int K>
+template <int DT, int K, bool PACK>
 __device__ __forceinline__ void march_plain(const FrameDesc &f, const DevBrick &b, float dx, float dy, float dz,
                                             float idx, float idy, float idz, float t0, float dt, float idt,
                                             float4 &acc, bool &done)
@@ -853,7 +915,7 @@ __device__ __forceinline__ void march_plain(const FrameDesc &f, const DevBrick &
     const VoxLattice L = vox_lattice(b, f.origx, f.origy, f.origz, dx, dy, dz, t0, dt);
     for (int i = cfg_first_ge(t0, dt, idt, tin); i < i1; i += K) {
         float s[K];
-        sample_run<DT, K>(b, L, (float) i, s);
+        sample_run<DT, K, PACK>(b, L, (float) i, s);
         if (composite_run<K>(f, s, i1 - i, f.alpha, f.term_alpha, acc)) {
             done = true;
             return;
@@ -1008,7 +1070,7 @@ __device__ __forceinline__ void march_runs(const FrameDesc &f, const DevBrick &b
             if (!__any_sync(kFullWarp, len > 0)) break;
             if (len == 0) continue;
             float s[K];
-            sample_run<DT, K>(b, L, (float) start, s);
+            sample_run<DT, K, false>(b, L, (float) start, s);
             if (composite_run<K>(f, s, len, opac, term, acc)) {
                 done = true;
                 nr = 0;
@@ -1155,7 +1217,7 @@ __device__ __forceinline__ float4 ray_cfg(const FrameDesc &f, int i, int j, bool
         } else if (SKIP && empty != nullptr) {
             march_runs<DT, K, PARK>(f, b, empty, runs, in, ray, acc, done);
         } else if (in) {
-            march_plain<DT, K>(f, b, ray[kDx], ray[kDy], ray[kDz], ray[kIdx], ray[kIdy], ray[kIdz], ray[kT0], ray[kDt],
+            march_plain<DT, SKIP ? K : kPlainK, !SKIP>(f, b, ray[kDx], ray[kDy], ray[kDz], ray[kIdx], ray[kIdy], ray[kIdz], ray[kT0], ray[kDt],
                                ray[kIdt], acc, done);
         }
     }
