@@ -96,8 +96,9 @@ typedef enum { IVR_SKIP_NONE = 0, IVR_SKIP_GRID = 1, IVR_SKIP_LEARNED = 2 } ivr_
 /* The order in which a CONFIG launch hands its 8x4 pixel tiles to warps.
  * IVR_TILES_COST (with a skipping grid): costliest first, by an estimate
  * from a walk of each tile's corner rays over the macrocell grid, so that the
- * launch does not end on a long tile drawn late.  The order never changes
- * a pixel. */
+ * launch does not end on a long tile drawn late.  A hint: frames of fewer
+ * than 8 tiles per resident warp (24,320 on 152 SMs) are handed out in row
+ * order all the same.  The order never changes a pixel. */
 typedef enum { IVR_TILES_RASTER = 0, IVR_TILES_COST = 1 } ivr_tile_order;
 
 /* How a frame is sampled.
@@ -275,10 +276,10 @@ int ivr_batch_free(ivr_batch *batch);
 int ivr_batch_clear(ivr_batch *batch);
 int ivr_batch_add(ivr_batch *batch, ivr_view *view, ivr_tf *tf, float *rgba32_dev, uint8_t *rgba8_dev);
 int ivr_batch_render(ivr_batch *batch, int use_graph, void *stream);
-/* Times every kernel variant (warp tiles 8x4, 4x8, 16x2; one or two
- * samples per loop iteration) on the filled batch and keeps the fastest.
- * variant (nullable) receives its index, ms_per_variant (nullable, 6 floats)
- * the timings. */
+/* Times every kernel variant (warp tiles 8x4, 4x8, 16x2; one sample per loop
+ * iteration, or four of u8 and u16 and two of f32) on the filled batch and
+ * keeps the fastest.  variant (nullable) receives its index, ms_per_variant
+ * (nullable, 6 floats) the timings. */
 int ivr_batch_autotune(ivr_batch *batch, void *stream, int *variant, float *ms_per_variant);
 int ivr_batch_set_variant(ivr_batch *batch, int variant);
 

@@ -47,8 +47,9 @@ def config_params(step=0.5, term_alpha=0.99, skip=True, tile=(1, 1), judge_strid
     """Benchmark sampling: true trilinear, ``step`` voxels, early termination.
     ``skip``: True/False for the exact grid or none, or a SKIP_* value
     (SKIP_LEARNED judges 1 in ``judge_stride`` tiles at ``judge_tol``).
-    ``tiles``: TILES_COST hands out the costliest tiles first (with a
-    skipping grid), TILES_RASTER in row order; the image is the same."""
+    ``tiles``: TILES_COST hands out the costliest tiles of large frames
+    first (with a skipping grid), TILES_RASTER in row order; the image is
+    the same."""
     p = RenderParams()
     _lib.load().ivr_params_config(ctypes.byref(p))
     p.step = step
