@@ -29,7 +29,9 @@ constexpr int kThreads = 128;
 // the start of the sweep K = 2 with 9 blocks): u16 learned 1024^3 at
 // 1920x1080 462, 368, 341, 368 (556); u16 without skipping 266, 218, 198,
 // 200 (368); u8 128^3 at 256x256 69, 56, 51, 51 (80); f32 (four registers a
-// voxel pair) 512^3 at 1024x1024 392, 342, 357, 352 (395).  The batched
+// voxel pair) 512^3 at 1024x1024 392, 342, 357, 352 (395); with the edges
+// clamped as they are now learned 328 and 356 at K = 6 and 8, f32 333 and 351
+// at K = 4 and 6.  The batched
 // kernel reads its frames from global memory and has no tail: there more
 // warps win (32 f32 frames of a 512^3 volume: 3.67 ms at K = 2 with 8 blocks,
 // 3.74 with 9, 3.92 with 7; 20 u16 frames 2.53 ms at K = 4 with 8, 3.06 with
@@ -1004,9 +1006,9 @@ template <> struct Ray<true> {
 // Every lane of the warp calls this (`in` false: without a ray), and the
 // loops are the warp's, so that lanes which leave a step early wait for the
 // others instead of taking the next step on their own (that took twice the
-// time).  Bound by the latency of the longest rays: of a 354 us f32 frame
-// (512^3, 1024x1024) the SMs have work for about 70%, with 43% of all issue
-// slots used.
+// time).  Bound by the latency of the longest rays: of a 317 us launch (384^3
+// f32, 2x2x2 bricks, 1024x1024) the SMs have work for 86%, and use 56% of
+// their issue slots meanwhile.
 template <int DT, int K, bool PARK>
 __device__ __forceinline__ void march_runs(const FrameDesc &f, const DevBrick &b, const uint8_t *empty,
                                            unsigned *runs, bool in, const Ray<PARK> &ray, float4 &acc, bool &done)
@@ -1752,7 +1754,7 @@ cudaError_t launch_dt(const FrameDesc &f, float4 *o32, uchar4 *o8, cudaStream_t 
 // persistent launch.  Frame descriptors are in device memory (uploaded with
 // the batch); a warp's ticket is a global tile number, mapped to its frame by
 // a binary search over the frames' first tiles.  Warp tiles are TW x (32/TW)
-// pixels; PAIR takes two samples per loop iteration.
+// pixels; PAIR takes batch_k samples per loop iteration, else one.
 template <int DT, int TW, bool PAIR>
 __global__ void __launch_bounds__(kThreads, kBatchBlocksPerSm)
     march_batch_kernel(const BatchHeader *__restrict__ hdr, const BatchItem *__restrict__ items,
