@@ -8,6 +8,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -460,29 +461,34 @@ bool learned_rejected(ivr_volume::TfGrid *g)
     return g->rejected;
 }
 
-// Whether a plain CONFIG frame's launch on s may begin while the one before
-// it ends (launch_march's early).  All it reads before it waits for that launch
-// are the volume, the LUT and the grid, so the grid's build has to lie before
-// the launch it overlaps: the first launch on each stream after a build waits
-// for it, and those that follow may be early.  (Streams by their id: a handle
-// may be a new stream's.)  Not in a stream capture.
-int may_be_early(ivr_ctx *c, ivr_volume::TfGrid *grid, cudaStream_t s, bool *early)
+// Before a CONFIG frame's first launch on s: the stream waits for the builds of
+// the grids that the frame reads (null: none), which other streams may still
+// be running, once per stream and build.  *early: whether a plain frame's launch
+// may begin while the one before it ends (launch_march's early).  All that it
+// reads before it waits for that launch are the volume, the LUT and the grid,
+// so the build has to lie before the launch it overlaps: the first launch on a
+// stream after a build is never early, those that follow may be.  (Streams by
+// their id: a handle may be a new stream's.)  A stream capture takes no event
+// from outside: there the frames are neither early nor made to wait, and a
+// graph is launched once the grids that its frames read are built.
+int after_builds(ivr_ctx *c, cudaStream_t s, std::initializer_list<ivr_volume::TfGrid *> grids, bool *early)
 {
     *early = false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(c, cudaStreamIsCapturing(s, &cap));
     if (cap != cudaStreamCaptureStatusNone) return IVR_OK;
-    if (grid) {
+    bool waited = false;
+    for (auto *g : grids) {
+        if (!g) continue;
         unsigned long long id = 0;
         CK(c, cudaStreamGetId(s, &id));
-        auto &seen = grid->after_build;
-        if (std::find(seen.begin(), seen.end(), id) == seen.end()) {
-            CK(c, cudaStreamWaitEvent(s, grid->built, 0));
-            if (seen.size() < 64) seen.push_back(id);
-            return IVR_OK;
-        }
+        auto &seen = g->after_build;
+        if (std::find(seen.begin(), seen.end(), id) != seen.end()) continue;
+        CK(c, cudaStreamWaitEvent(s, g->built, 0));
+        if (seen.size() < 64) seen.push_back(id);
+        waited = true;
     }
-    *early = true;
+    *early = !waited;
     return IVR_OK;
 }
 
@@ -704,11 +710,11 @@ int render_window(ivr_view *view, ivr_tf *tf, int x, int y, int w, int h, int si
         if (rc) return rc;
     }
     bool early = false;
-    if (f.preset == IVR_PRESET_CONFIG && !touched && !judged) {
-        rc = may_be_early(c, grid, s, &early);
+    if (f.preset == IVR_PRESET_CONFIG) {
+        rc = after_builds(c, s, {grid, exact}, &early);
         if (rc) return rc;
     }
-    rc = launch_view(view, f, o32, o8, s, early);
+    rc = launch_view(view, f, o32, o8, s, early && !touched && !judged);
     if (rc == IVR_OK && judged) {
         const cudaError_t je = launch_judge_compare(f, (const uchar4 *) o8, (const float4 *) o32, s);
         if (je != cudaSuccess) rc = cuda_fail(c, je, "judge compare launch");
