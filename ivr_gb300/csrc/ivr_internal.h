@@ -152,6 +152,32 @@ struct HostBrick {
 
 size_t dtype_size(int dtype);
 
+#ifdef __CUDACC__
+#define IVR_HD __host__ __device__ __forceinline__
+#else
+#define IVR_HD inline
+#endif
+// A sample's LUT index before lut_at clamps it: x, its scaled value as an int
+// (the conversion saturates), less the LUT's offset, modulo 2^32.
+IVR_HD int lut_index(int x, int off) { return (int) ((unsigned) x - (unsigned) off); }
+// The LUT entries lo..hi that samples of a macrocell can index, from the
+// scaled minimum and maximum of its voxels as ints: samples lie between the
+// voxels up to rounding, so one entry more at each end.  In 64 bits, since
+// voxels beyond the ints (infinities among them) saturate: in 32 bits the one
+// entry more overflows, and the compiler, which may take it that it does not,
+// moves the addition out of the clamp that keeps the index in the LUT.  Where
+// lut_index wraps, the entries are all.
+struct LutRange {
+    int lo, hi;
+};
+IVR_HD LutRange lut_range(int x0, int x1, int off, int n)
+{
+    const long long i0 = (long long) x0 - off, i1 = (long long) x1 - off, top = n - 1;
+    if (i0 < -2147483647LL - 1 || i1 > 2147483647LL) return LutRange{0, n - 1};
+    const long long lo = i0 - 1 < 0 ? 0 : i0 - 1, hi = i1 + 1 < 0 ? 0 : i1 + 1;
+    return LutRange{(int) (lo < top ? lo : top), (int) (hi < top ? hi : top)};
+}
+
 // kernels (ivr_kernels.cu)
 cudaError_t launch_byteswap(void *data, long long n, int elem, cudaStream_t s);
 cudaError_t launch_gather_brick(const void *src, int gw, int gh, int gd, void *dst, int sx, int sy, int sz,

@@ -443,9 +443,8 @@ cudaError_t macrocells_dt(const T *data, int nx, int ny, int nz, int cell, float
     return cudaGetLastError();
 }
 
-// A cell is transparent when no LUT entry its samples can index has
-// non-zero opacity.  Samples lie in [min, max] of the cell's voxels up to
-// rounding, so the index range is widened by one on each side.
+// A cell is transparent when no LUT entry its samples can index (lut_range)
+// has non-zero opacity.
 // nzprefix[i] = number of entries in [0, i) with non-zero opacity.
 // Writes kDistCap for a transparent cell and 0 for the others.  In the same
 // pass (opac non-null), the tile cost estimate's input: 255 sqrt(mean LUT
@@ -456,13 +455,12 @@ __global__ void empty_kernel(const float *mc, int ncell, const int *nzprefix, co
                              int lut_off, float lut_scale, uint8_t *dist, uint8_t *opac)
 {
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) {
-        const int i0 = (int) (mc[2 * c] * lut_scale) - lut_off, i1 = (int) (mc[2 * c + 1] * lut_scale) - lut_off;
-        const int lo = min(max(i0 - 1, 0), lut_n - 1);
-        const int hi = min(max(i1 + 1, 0), lut_n - 1);
-        dist[c] = (nzprefix[hi + 1] - nzprefix[lo]) == 0 ? (uint8_t) kDistCap : 0;
+        const int x0 = __float2int_rz(mc[2 * c] * lut_scale), x1 = __float2int_rz(mc[2 * c + 1] * lut_scale);
+        const LutRange r = lut_range(x0, x1, lut_off, lut_n);
+        dist[c] = (nzprefix[r.hi + 1] - nzprefix[r.lo]) == 0 ? (uint8_t) kDistCap : 0;
         if (opac) {
-            const int a = min(max(i0, 0), lut_n - 1);
-            const int b = min(max(i1, a), lut_n - 1);
+            const int a = min(max(lut_index(x0, lut_off), 0), lut_n - 1);
+            const int b = min(max(lut_index(x1, lut_off), a), lut_n - 1);
             const double mean = (aprefix[b + 1] - aprefix[a]) / (double) (b - a + 1);
             const float q = sqrtf(fminf(fmaxf((float) mean, 0.0f), 1.0f)) * 255.0f + 0.5f;
             opac[c] = (uint8_t) min((int) q, 255);

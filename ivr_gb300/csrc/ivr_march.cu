@@ -674,7 +674,7 @@ template <int TF>
 __device__ __forceinline__ float4 ref_entry(const FrameDesc &f, float s)
 {
     if (TF == IVR_TF_RGBBLEND) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    return lut_at(f, (int) s - (TF == IVR_TF_BLEND ? 0 : f.lut_off));
+    return lut_at(f, lut_index((int) s, TF == IVR_TF_BLEND ? 0 : f.lut_off));
 }
 
 // The ray's iend samples by sample_ref itself, one by one: rays on which
@@ -842,7 +842,7 @@ __device__ __forceinline__ bool composite_run(const FrameDesc &f, const float (&
 {
     float4 e[K];
 #pragma unroll
-    for (int k = 0; k < K; k++) e[k] = lut_at(f, (int) (s[k] * f.lut_scale) - f.lut_off);
+    for (int k = 0; k < K; k++) e[k] = lut_at(f, lut_index((int) (s[k] * f.lut_scale), f.lut_off));
 #pragma unroll
     for (int k = 0; k < K; k++) {
         if (k >= n) break;
@@ -1646,7 +1646,7 @@ __global__ void __launch_bounds__(kThreads, kPeakBlocksPerSm) sample_peak_kernel
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (int i = 0; i < steps; i++) {
         const float s = sample_layout<DT, LAYOUT>(b, tex, x, y, z);
-        const float4 e = lut_at(f, (int) (s * f.lut_scale) - f.lut_off);
+        const float4 e = lut_at(f, lut_index((int) (s * f.lut_scale), f.lut_off));
         const float wgt = (1.0f - acc.w) * (e.w * f.alpha);
         acc.x = fmaf(wgt, e.x, acc.x);
         acc.y = fmaf(wgt, e.y, acc.y);

@@ -119,10 +119,9 @@ __global__ void cell_features_kernel(const float *mc, const float *hist, int nce
         for (int k = 0; k < 16; k++) x[10 + k] = __float2bfloat16(knots[k]);
         for (int k = kMlpFeatures; k < kMlpIn; k++) x[k] = __float2bfloat16(0.0f);
         if (targets) {
-            int a = min(max((int) (lo * lut_scale) - 1 - lut_off, 0), lut_n - 1);
-            int b = min(max((int) (hi * lut_scale) + 1 - lut_off, 0), lut_n - 1);
+            const LutRange r = lut_range(__float2int_rz(lo * lut_scale), __float2int_rz(hi * lut_scale), lut_off, lut_n);
             float m = 0.0f;
-            for (int i = a; i <= b; i++) m = fmaxf(m, lut[i].w);
+            for (int i = r.lo; i <= r.hi; i++) m = fmaxf(m, lut[i].w);
             targets[c] = m;
         }
     }

@@ -280,9 +280,9 @@ __global__ void __launch_bounds__(kRows) mlp_tc_kernel(MlpDev w, const bf16 *X, 
             if (GRID) {
                 // learned transparency, certified by the exact empty-cell test
                 const bool learned = yv + g.margin <= 0.0f;
-                const int a = min(max((int) (lo * g.lut_scale) - 1 - g.lut_off, 0), g.lut_n - 1);
-                const int b = min(max((int) (hi * g.lut_scale) + 1 - g.lut_off, 0), g.lut_n - 1);
-                const bool exact = (g.nzprefix[b + 1] - g.nzprefix[a]) == 0;
+                const LutRange r = lut_range(__float2int_rz(lo * g.lut_scale), __float2int_rz(hi * g.lut_scale),
+                                             g.lut_off, g.lut_n);
+                const bool exact = (g.nzprefix[r.hi + 1] - g.nzprefix[r.lo]) == 0;
                 g.dist[row] = (learned && (exact || !g.certify)) ? (uint8_t) kDistCap : 0;
                 ncells++;
                 nexact += exact;
