@@ -271,6 +271,7 @@ int alloc_bricks(ivr_volume *v)
     if (qneed > v->quad_cap || qneed == 0) free_quad_block(v);
     cudaError_t e = cudaMalloc(&v->brick_block, need);
     if (e != cudaSuccess && v->quad_block) {
+        cudaGetLastError();  // or the launches that follow would report it
         free_quad_block(v);
         e = cudaMalloc(&v->brick_block, need);
     }

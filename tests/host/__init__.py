@@ -26,7 +26,7 @@ def load(directory) -> ctypes.CDLL:
     for name in ("fake_in_use", "fake_mallocs", "fake_launches", "fake_early"):
         getattr(lib, name).restype = ctypes.c_size_t
     lib.fake_capacity.argtypes = [ctypes.c_size_t]
-    lib.fake_fail_malloc.argtypes = lib.fake_fail_launch.argtypes = [ctypes.c_long]
+    lib.fake_fail_malloc.argtypes = lib.fake_fail_more.argtypes = lib.fake_fail_launch.argtypes = [ctypes.c_long]
     lib.cudaStreamCreateWithFlags.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_uint]
     lib.cudaDeviceSynchronize.argtypes = []
     lib.cudaStreamBeginCapture.argtypes = [ctypes.c_void_p, ctypes.c_int]

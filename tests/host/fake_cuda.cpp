@@ -47,7 +47,7 @@ struct State {
     std::string first;              // the first of them
     std::map<void *, size_t> live;  // device allocations
     size_t in_use = 0, capacity = ~(size_t) 0;
-    long mallocs = 0, fail_malloc = -1, fail_launch = -1, launches = 0, early = 0;
+    long mallocs = 0, fail_malloc = -1, fail_more = 0, fail_launch = -1, launches = 0, early = 0;
     cudaError_t last = cudaSuccess;
 } g;
 
@@ -134,6 +134,7 @@ void fake_reset(void)
     g.readers.clear();
     g.mallocs = g.launches = g.early = 0;
     g.fail_malloc = g.fail_launch = -1;
+    g.fail_more = 0;
     g.capacity = ~(size_t) 0;
     g.last = cudaSuccess;
 }
@@ -144,7 +145,9 @@ long fake_mallocs(void) { return g.mallocs; }
 long fake_launches(void) { return g.launches; }
 long fake_early(void) { return g.early; }
 void fake_capacity(size_t n) { g.capacity = n; }
-void fake_fail_malloc(long n) { g.fail_malloc = n; }  // the n-th from now (0: the next)
+// the n-th allocation from now fails (0: the next one), and `more` behind it
+void fake_fail_malloc(long n) { g.fail_malloc = n; }
+void fake_fail_more(long n) { g.fail_more = n; }
 void fake_fail_launch(long n) { g.fail_launch = n; }
 
 cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
@@ -161,7 +164,9 @@ const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAlloc
 cudaError_t cudaMalloc(void **p, size_t n)
 {
     g.mallocs++;
-    if ((g.fail_malloc >= 0 && g.fail_malloc-- == 0) || n > g.capacity - std::min(g.capacity, g.in_use))
+    const bool fails = g.fail_malloc == 0;
+    if (g.fail_malloc > 0 || (fails && g.fail_more-- == 0)) g.fail_malloc--;
+    if (fails || n > g.capacity - std::min(g.capacity, g.in_use))
         return error(cudaErrorMemoryAllocation);
     if (posix_memalign(p, 512, (n + 511) / 512 * 512)) return error(cudaErrorMemoryAllocation);
     memset(*p, 0, n);
