@@ -294,6 +294,21 @@ int alloc_bricks(ivr_volume *v)
     return alloc_each(c, arrays);
 }
 
+// The voxels, macrocells and copies of bricks that have their memory.
+int fill_bricks(ivr_volume *v)
+{
+    ivr_ctx *c = v->ctx;
+    for (auto &b : v->bricks) {
+        if (b.owns)
+            CK(c, launch_gather_brick(v->d_full, v->w, v->h, v->d, b.data, b.sx, b.sy, b.sz, b.lw, b.lh, b.ld,
+                                      (int) dtype_size(v->dtype), 0));
+        CK(c, launch_macrocells(b.data, v->dtype, b.lw, b.lh, b.ld, b.cell, b.mc_minmax, b.mcx, b.mcy, b.mcz, 0));
+        if (b.quad) CK(c, launch_quads(b.data, v->dtype, b.lw, b.lh, b.ld, b.quad, 0));
+    }
+    CK(c, cudaDeviceSynchronize());
+    return IVR_OK;
+}
+
 int setup_bricks(ivr_volume *v, int py, int px, int pz, int overlap)
 {
     ivr_ctx *c = v->ctx;
@@ -318,16 +333,9 @@ int setup_bricks(ivr_volume *v, int py, int px, int pz, int overlap)
         b.mcy = (b.lh - 2) / b.cell + 1;
         b.mcz = (b.ld - 2) / b.cell + 1;
     }
-    const int rc = alloc_bricks(v);
+    int rc = alloc_bricks(v);
+    if (rc == IVR_OK) rc = fill_bricks(v);
     if (rc) { free_bricks(v); return rc; }
-    for (auto &b : v->bricks) {
-        if (b.owns)
-            CK(c, launch_gather_brick(v->d_full, v->w, v->h, v->d, b.data, b.sx, b.sy, b.sz, b.lw, b.lh, b.ld,
-                                      (int) dtype_size(v->dtype), 0));
-        CK(c, launch_macrocells(b.data, v->dtype, b.lw, b.lh, b.ld, b.cell, b.mc_minmax, b.mcx, b.mcy, b.mcz, 0));
-        if (b.quad) CK(c, launch_quads(b.data, v->dtype, b.lw, b.lh, b.ld, b.quad, 0));
-    }
-    CK(c, cudaDeviceSynchronize());
     v->py = py; v->px = px; v->pz = pz; v->overlap = overlap;
     return IVR_OK;
 }

@@ -1,5 +1,5 @@
-"""CPU: brick set-up on a device that runs out of memory: a refusal leaves
-nothing behind, and no call reports another's failure."""
+"""CPU: brick set-up on a device that runs out of memory, and with launches
+that fail: a refusal leaves nothing behind, and no call reports another's failure."""
 import ctypes
 
 import numpy as np
@@ -73,6 +73,30 @@ def test_allocations_that_fail(lib, grid, first, more):
     elif first + more == 0:  # (the kept copies' block is given back, and asked for again)
         assert v.quad_bytes() == copies
     assert ctx.mem_used == empty + m + v.quad_bytes()
+    frame(ctx, v)
+    v.free()
+    ctx.close()
+    assert lib.fake_in_use() == 0
+
+
+@pytest.mark.parametrize("n", range(25))
+def test_launches_that_fail(lib, n):
+    """The set-up of eight bricks has 24 launches: one fails, no brick is left
+    that was not filled, and the next set-up is whole."""
+    lib.fake_reset()
+    ctx = HostContext(lib)
+    v = ctx.load_volume(VOL)
+    empty = ctx.mem_used - sum(needed((1, 1, 1)))
+    lib.fake_fail_launch(n)
+    rc = try_bricks(v, (2, 2, 2))
+    lib.fake_fail_launch(-1)
+    assert (rc != 0) == (n < 24)
+    if rc:
+        assert rc == -2 and ctx.mem_used == empty and v.quad_bytes() == 0
+        with pytest.raises(IvrError):
+            frame(ctx, v)
+        assert try_bricks(v, (2, 2, 2)) == 0
+    assert ctx.mem_used == empty + sum(needed((2, 2, 2)))
     frame(ctx, v)
     v.free()
     ctx.close()
