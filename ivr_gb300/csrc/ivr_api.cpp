@@ -269,29 +269,33 @@ int alloc_bricks(ivr_volume *v)
     for (const auto &a : arrays) (a.optional ? quads : must).push_back(a);
     const size_t need = block_bytes(must), qneed = block_bytes(quads);
     if (qneed > v->quad_cap || qneed == 0) free_quad_block(v);
-    cudaError_t e = cudaMalloc(&v->brick_block, need);
-    if (e != cudaSuccess && v->quad_block) {
-        cudaGetLastError();  // or the launches that follow would report it
+    // (a refused allocation's error is taken back at once: the launches that
+    // follow report what is left of it)
+    auto block = [](void **p, size_t bytes) {
+        if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+        cudaGetLastError();
+        *p = nullptr;
+        return false;
+    };
+    bool placed = block(&v->brick_block, need);
+    if (!placed && v->quad_block) {
         free_quad_block(v);
-        e = cudaMalloc(&v->brick_block, need);
+        placed = block(&v->brick_block, need);
     }
-    if (e != cudaSuccess) v->brick_block = nullptr;
-    if (e == cudaSuccess && qneed && !v->quad_block) {
+    if (!placed) return alloc_each(c, arrays);
+    place(must, v->brick_block);
+    for (const auto &a : must) c->used += a.bytes;
+    // Where the copies have no block, with or without the spare slabs, those
+    // that fit by themselves are kept: what a layout must have is placed.
+    if (qneed && !v->quad_block) {
         const size_t spare = c->budget ? 0 : kQuadSpare * quad_bytes(v->dtype, v->w, v->h, 1);
-        e = cudaMalloc(&v->quad_block, qneed + spare);
-        if (e == cudaSuccess) v->quad_cap = qneed + spare;
-        else v->quad_block = nullptr;
+        if (block(&v->quad_block, qneed + spare)) v->quad_cap = qneed + spare;
+        else if (spare && block(&v->quad_block, qneed)) v->quad_cap = qneed;
+        else return alloc_each(c, quads);
     }
-    if (e == cudaSuccess) {
-        place(must, v->brick_block);
-        if (qneed) place(quads, v->quad_block);
-        c->used = used;
-        return IVR_OK;
-    }
-    cudaGetLastError();
-    cudaFree(v->brick_block);
-    v->brick_block = nullptr;
-    return alloc_each(c, arrays);
+    if (qneed) place(quads, v->quad_block);
+    for (const auto &a : quads) c->used += a.bytes;
+    return IVR_OK;
 }
 
 // The voxels, macrocells and copies of bricks that have their memory.

@@ -1,5 +1,7 @@
-"""CPU: brick set-up on a device that runs out of memory, and with launches
-that fail: a refusal leaves nothing behind, and no call reports another's failure."""
+"""CPU: brick set-up on a device that runs out of memory, allocation by
+allocation and at every capacity, and with launches that fail: what is needed
+is placed while it fits, the corner-packed copies are left out where they do
+not, a refusal leaves nothing behind, and no call reports another's failure."""
 import ctypes
 
 import numpy as np
@@ -77,6 +79,36 @@ def test_allocations_that_fail(lib, grid, first, more):
     v.free()
     ctx.close()
     assert lib.fake_in_use() == 0
+
+
+@pytest.mark.parametrize("grid", [(2, 2, 2), (1, 1, 4), (3, 1, 2)])
+def test_every_capacity(lib, grid):
+    lib.fake_reset()
+    must, copies = needed(grid)
+    served = 0
+    for extra in range(0, copies + copies // 4, 4096):
+        lib.fake_capacity(1 << 40)
+        ctx = HostContext(lib)
+        base = lib.fake_in_use() + VOL.nbytes
+        v = ctx.load_volume(VOL)
+        lib.fake_capacity(base + must + extra)
+        rc = try_bricks(v, grid)
+        assert lib.cudaGetLastError() == 0
+        # what must be fits (but for the arrays' alignment)
+        if extra >= 512 * 2 * np.prod(grid):
+            assert rc == 0, extra
+        if rc == 0:
+            got = v.quad_bytes()
+            assert served <= got <= extra  # more room, more copies
+            served = got if got == copies else 0
+            assert ctx.mem_used <= lib.fake_in_use()
+        lib.fake_capacity(1 << 40)
+        if rc == 0:
+            frame(ctx, v)
+        v.free()
+        ctx.close()
+        assert lib.fake_in_use() == 0
+    assert served == copies
 
 
 @pytest.mark.parametrize("n", range(25))
