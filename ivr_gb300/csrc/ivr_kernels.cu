@@ -253,9 +253,34 @@ __global__ void __launch_bounds__(1024) hist_kernel(const T *__restrict__ data, 
     }
 }
 
+// The same for volumes of few voxels and as many bins as a block's static
+// shared memory has counters: a counter a bin, a voxel a step, small blocks.
+// What bounds it are the launch and the counters' clearing and adding up, which
+// hist_kernel's large blocks, copies and vectors only make longer.  Kernel
+// alone, this and hist_kernel: 32^3 u8, 256 bins 2.1 and 3.9 us, 116^3 f32, 256
+// bins 3.4 and 5.7, 160^3 u16, 4096 bins 10.4 and 8.7.
+constexpr int kHistFewBins = 12288;
+template <typename T>
+__global__ void __launch_bounds__(512) hist_few_kernel(const T *__restrict__ data, long long n, MinArg mn, int hsize,
+                                                       int *hist)
+{
+    __shared__ int sh[kHistFewBins];
+    for (int b = threadIdx.x; b < hsize; b += blockDim.x) sh[b] = 0;
+    __syncthreads();
+    const float fmin = mn.dev ? __ldg(mn.dev) : mn.v;
+    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
+        const int b = (int) ((float) __ldg(data + i) - fmin);
+        if ((unsigned) b < (unsigned) hsize) atomicAdd(&sh[b], 1);
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < hsize; b += blockDim.x)
+        if (sh[b]) atomicAdd(&hist[b], sh[b]);
+}
+
 // The same with the counters in global memory: for more bins than two ranges
 // hold (float volumes of a wide range), and for volumes too small to pay for
-// clearing and adding up shared counters.
+// clearing and adding up the shared counters of more bins than hist_few_kernel
+// takes.
 template <typename T>
 __global__ void hist_global_kernel(const T *__restrict__ data, long long n, MinArg mn, int hsize, int *hist)
 {
@@ -635,10 +660,14 @@ constexpr int kHistRanges = 2;              // ranges before the counters move t
                                             // at four (229,375 bins, 256^3 f32 voxels) a call
                                             // took 130 us against 88 in global memory, at two
                                             // (65,536 bins, 256^3 u16) 75 against 87
-constexpr int kHistSmall = 128;             // voxels per bin below which global counters win:
-                                            // 256 bins, u8: 32^3 (128 a bin) 25.5 us shared, 24.4
-                                            // global, 48^3 (432) 25.7 and 33.0; 65,536 bins, u16:
-                                            // 160^3 (62) 52 and 47, 256^3 (256) 75 and 87
+constexpr long long kHistFew = 8192LL * 2 * kHistBlocks;  // voxels from which hist_kernel's blocks have
+                                                         // work for the time their counters take
+constexpr int kHistSmall = 128;             // voxels per bin below which global counters win, of more
+                                            // bins than hist_few_kernel takes: 65,536 bins, u16: 160^3
+                                            // (62 a bin) 52 us a call shared and 47 global, 256^3 (256)
+                                            // 75 and 87.  (With fewer bins they lose: voxels that crowd
+                                            // in one wait for each other.  80^3 u16 voxels, 60% of one
+                                            // value, 4096 bins: 151 us global, 4.2 in hist_few_kernel.)
 
 template <typename T>
 cudaError_t hist_launch(const T *data, long long n, MinArg mn, int hsize, int *hist, cudaStream_t s)
@@ -664,7 +693,11 @@ template <typename T>
 cudaError_t hist_dt(const T *data, long long n, MinArg mn, int hsize, int *hist, cudaStream_t s)
 {
     if (sizeof(T) < 4) hsize = std::min(hsize, 65536);  // integer voxels: the bins above stay empty
-    if (hsize > kHistRanges * kHistBins || n < (long long) kHistSmall * hsize) {
+    if (hsize <= kHistFewBins && n < kHistFew) {
+        hist_few_kernel<<<grid_for(n, 512, 2), 512, 0, s>>>(data, n, mn, hsize, hist);
+        return cudaGetLastError();
+    }
+    if (hsize > kHistRanges * kHistBins || (hsize > kHistFewBins && n < (long long) kHistSmall * hsize)) {
         hist_global_kernel<<<grid_for(n, 256), 256, 0, s>>>(data, n, mn, hsize, hist);
         return cudaGetLastError();
     }
