@@ -913,29 +913,32 @@ cudaError_t launch_gradient(const void *data, int dtype, int w, int h, int d, fl
     return cudaGetLastError();
 }
 
-// Corner-packed copy; bound by its stores (4x the brick).  A warp takes 32
-// elements of a row and walks kQuadRows rows, each voxel row loaded once for
+// Corner-packed copy; bound by its stores (4x the brick).  A thread walks
+// kQuadRows rows down its column (slab_block), each voxel row loaded once for
 // the two element rows it belongs to.  With a 64-bit division per index and
-// an element a thread it took 4.9 ms for 1024^3 u16 voxels (2.2 TB/s).
+// an element a thread it took 4.9 ms for 1024^3 u16 voxels (2.2 TB/s).  Narrow
+// bricks, u16, so, in whole warps a row and an element a thread: 8x1024x1024
+// voxels (x, y, z) 14, 45 and 26 us, 2x2048x2048 18, 173 and 16.
 constexpr int kQuadRows = 4;
 template <typename T, typename V>
-__global__ void __launch_bounds__(256) quad_kernel(const T *__restrict__ src, int nx, int ny, V *__restrict__ dst,
-                                                   unsigned bx, unsigned by)
+__global__ void __launch_bounds__(256) quad_kernel(const T *__restrict__ src, int nx, int ny, int nz,
+                                                   V *__restrict__ dst, unsigned bx, unsigned by)
 {
     const int qx = nx - 1, qy = ny - 1;
     const unsigned r = blockIdx.x / bx;
-    const int j = (int) (blockIdx.x % bx) * 32 + (threadIdx.x & 31);
-    const int i0 = ((int) (r % by) * 8 + (int) (threadIdx.x >> 5)) * kQuadRows;
-    const long long k = r / by;
-    if (j >= qx || i0 >= qy) return;
+    const int j = (int) (blockIdx.x % bx * blockDim.x + threadIdx.x);
+    const int i0 = (int) (r % by * blockDim.y + threadIdx.y) * kQuadRows;
+    const long long k = r / by * blockDim.z + threadIdx.z;
+    if (j >= qx || i0 >= qy || k >= nz) return;
     const T *p = src + (k * ny + i0) * nx + j;
     V *q = dst + (k * qy + i0) * qx + j;
     T a[kQuadRows + 1], b[kQuadRows + 1];
 #pragma unroll
-    for (int u = 0; u <= kQuadRows; u++) {  // past the last row: the last one again
-        const T *row = p + (long long) min(u, qy - i0) * nx;
-        a[u] = __ldg(row);
-        b[u] = __ldg(row + 1);
+    for (int u = 0; u <= kQuadRows; u++) {
+        const T *row = p + (long long) u * nx;
+        const bool in = i0 + u <= qy;
+        a[u] = in ? __ldg(row) : T(0);
+        b[u] = in ? __ldg(row + 1) : T(0);
     }
 #pragma unroll
     for (int u = 0; u < kQuadRows; u++) {
@@ -962,12 +965,13 @@ size_t quad_bytes(int dtype, int nx, int ny, int nz)
 
 cudaError_t launch_quads(const void *data, int dtype, int nx, int ny, int nz, void *quad, cudaStream_t s)
 {
-    const unsigned bx = (unsigned) (nx - 1 + 31) / 32, by = (unsigned) (ny - 1 + 8 * kQuadRows - 1) / (8 * kQuadRows);
-    const unsigned grid = (unsigned) ((unsigned long long) bx * by * nz);
+    const dim3 block = slab_block(nx - 1, (ny - 1 + kQuadRows - 1) / kQuadRows, 32);
+    const unsigned bx = (nx - 1 + block.x - 1) / block.x, by = (ny - 1 + block.y * kQuadRows - 1) / (block.y * kQuadRows);
+    const unsigned grid = (unsigned) ((unsigned long long) bx * by * ((nz + block.z - 1) / block.z));
     switch (dtype) {
-    case IVR_U8: quad_kernel<<<grid, 256, 0, s>>>((const uint8_t *) data, nx, ny, (uchar4 *) quad, bx, by); break;
-    case IVR_U16: quad_kernel<<<grid, 256, 0, s>>>((const uint16_t *) data, nx, ny, (ushort4 *) quad, bx, by); break;
-    case IVR_F32: quad_kernel<<<grid, 256, 0, s>>>((const float *) data, nx, ny, (float4 *) quad, bx, by); break;
+    case IVR_U8: quad_kernel<<<grid, block, 0, s>>>((const uint8_t *) data, nx, ny, nz, (uchar4 *) quad, bx, by); break;
+    case IVR_U16: quad_kernel<<<grid, block, 0, s>>>((const uint16_t *) data, nx, ny, nz, (ushort4 *) quad, bx, by); break;
+    case IVR_F32: quad_kernel<<<grid, block, 0, s>>>((const float *) data, nx, ny, nz, (float4 *) quad, bx, by); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -63,3 +63,51 @@ def test_gradient_takes_no_longer(ctx, shape):
         us[s] = device_us(lambda: v.gradient(out.data_ptr()))
         v.free()
     assert us[shape] < 2.0 * us[(256, 256, 128)], us
+
+
+@pytest.mark.parametrize("dtype", ["u8", "u16", "f32"])
+@pytest.mark.parametrize("shape,bricks", [((2, 2, 2), (1, 1, 1)), ((70, 2, 2), (1, 1, 2)), ((65, 4, 3), (2, 1, 1)),
+                                          ((9, 5, 6), (2, 2, 1)), ((7, 40, 5), (1, 1, 1)), ((33, 35, 33), (1, 1, 1)),
+                                          ((5, 3, 34), (1, 1, 1)), ((6, 38, 66), (1, 2, 1)), ((2, 260, 9), (3, 1, 1))])
+def test_corner_packed_copies(ctx, dtype, shape, bricks):
+    """Frames from the copies are those from the voxels."""
+    import torch
+    from ivr_gb300 import api, synth
+    from ivr_gb300.state import orbit_state
+    v = ctx.load_volume(volume(shape, dtype)).bricks(*bricks)
+    tf = ctx.transfer_function().set_lut(synth.ramp_tf(256), 0, 256.0 / 65536.0 if dtype == "u16" else 1.0)
+    frames = []
+    for on in (True, False):
+        v.quads(on)
+        assert (v.quad_bytes() > 0) == on
+        view = ctx.view().set(v, orbit_state(35.0, 25.0, 160, 120), api.config_params(step=0.1, term_alpha=2.0))
+        out = torch.full((120, 160, 4), -7.0, device="cuda")
+        view.render(tf, out.data_ptr())
+        torch.cuda.synchronize()
+        frames.append(out.cpu().numpy().view(np.uint32))
+        view.free()
+    v.free()
+    tf.free()
+    assert frames[1].any() and np.array_equal(*frames)
+
+
+def test_corner_packed_copies_take_no_longer(ctx):
+    """What the copies add to the set-up of a thin brick, against a cube's."""
+    import time
+    import torch
+    added = {}
+    for shape in ((512, 512, 128), (4096, 4096, 2)):
+        v = ctx.load_volume(np.zeros(shape, np.uint8))
+        took = {}
+        for on in (True, False):
+            v.quads(on)
+            t = []
+            for _ in range(9):
+                torch.cuda.synchronize()
+                a = time.perf_counter()
+                v.bricks(1, 1, 1)  # (ends with a synchronisation)
+                t.append(1e6 * (time.perf_counter() - a))
+            took[on] = np.median(t)
+        added[shape] = took[True] - took[False]
+        v.free()
+    assert added[(4096, 4096, 2)] < 2.0 * added[(512, 512, 128)] + 100.0, added
