@@ -229,10 +229,10 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
 // rounded to nearest (Markstein, "Computation of elementary functions on the
 // IBM RISC System/6000 processor", 1990, theorem on the final division step;
 // the two-word reciprocal is Brisebarre and Muller's, "Correctly rounded
-// multiplication by arbitrary precision constants", 2008).  Neither bound
-// holds near the ends of the exponent range: callers pass 0 < |x| in
-// [kDivMin, kDivMax] or x = 0, and divisors in the same range.
-constexpr float kDivMin = 8.673617379884035e-19f, kDivMax = 1.152921504606847e18f;  // 2^-60, 2^60
+// multiplication by arbitrary precision constants", 2008).  Both hold while
+// nothing overflows, the quotient is normal and the remainder, a multiple of
+// 2^-47 |x|, is no finer than floats are: for x = 0 and |x| in [2^-73, 2^98]
+// with c in [2^-16, 2^40], which is what ref_fast lets through.
 struct FixedDiv {
     F2 mc, h, l;  // -c, 1/c, the rest of 1/c, for both lanes
     __device__ __forceinline__ explicit FixedDiv(float d)
@@ -250,24 +250,31 @@ struct FixedDiv {
 };
 
 // Whether every division that sample_ref makes along the ray is one that
-// FixedDiv rounds as IEEE division does.  The positions x = o + d t are
-// compared with a brick edge and cell corners; where those, or o, are at
-// least 2^-30, the difference of two floats near each other is a multiple of
-// the smaller one's last place, so it is 0 or at least 2^-57.  An edge at 0
-// (inner bricks) seen from o = 0 needs d t away from 0 as well.
-__device__ __forceinline__ bool ref_fast_axis(float o, float d, float bmin, float extent, float tin)
+// FixedDiv rounds as IEEE division does.  The divisors are the brick's extents
+// and dims.  The positions x = o + d t are compared with a brick edge and cell
+// corners (at least 2^-32 where they are not 0); where the edge or o is at least
+// 2^-30, the difference of two floats near each other is a multiple of the
+// smaller one's last place, so it is 0 or at least 2^-57.  An edge at 0 (inner
+// bricks) seen from o = 0 needs d t away from 0 as well.  The last division's
+// dividend is such a difference times the extent: 2^-73 at least.  Positions are
+// below 2^58 (t is at most 2^17), times an extent 2^98.
+constexpr float kRefNear = 9.313225746154785e-10f, kRefFar = 1.099511627776e12f;  // 2^-30, 2^40
+constexpr float kRefThin = 1.52587890625e-5f;                                     // 2^-16
+constexpr int kRefDim = 1 << 16;
+__device__ __forceinline__ bool ref_fast_axis(float o, float d, float bmin, float extent, int dim, float tin)
 {
-    const float tiny = 9.313225746154785e-10f, huge = 1.099511627776e12f;  // 2^-30, 2^40
-    if (!(fabsf(o) <= huge && fabsf(d) <= huge && extent >= tiny && extent <= huge && fabsf(bmin) <= huge)) return false;
-    if (fabsf(bmin) >= tiny) return true;
+    if (!(fabsf(o) <= kRefFar && fabsf(d) <= kRefFar && extent >= kRefThin && extent <= kRefFar &&
+          fabsf(bmin) <= kRefFar && dim <= kRefDim))
+        return false;
+    if (fabsf(bmin) >= kRefNear) return true;
     if (bmin != 0.0f) return false;
-    if (fabsf(o) >= tiny) return true;
-    return o == 0.0f && (d == 0.0f || (fabsf(d) >= tiny && tin >= 1.0e-6f));
+    if (fabsf(o) >= kRefNear) return true;
+    return o == 0.0f && (d == 0.0f || (fabsf(d) >= kRefNear && tin >= 1.0e-6f));
 }
 __device__ __forceinline__ bool ref_fast(const FrameDesc &f, const DevBrick &b, float dx, float dy, float dz, float tin)
 {
-    return fabsf(tin) <= 65536.0f && ref_fast_axis(f.origx, dx, b.bminx, b.w, tin) &&
-           ref_fast_axis(f.origy, dy, b.bminy, b.h, tin) && ref_fast_axis(f.origz, dz, b.bminz, b.d, tin);
+    return fabsf(tin) <= 65536.0f && ref_fast_axis(f.origx, dx, b.bminx, b.w, b.nx, tin) &&
+           ref_fast_axis(f.origy, dy, b.bminy, b.h, b.ny, tin) && ref_fast_axis(f.origz, dz, b.bminz, b.d, b.nz, tin);
 }
 
 // A ray's REF sampler in one brick: sample_ref with its nine divisions, all
