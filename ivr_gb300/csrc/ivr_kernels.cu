@@ -601,20 +601,19 @@ __device__ __forceinline__ unsigned q8k(float v)
 // HBM-bound; four floats in, one 32-bit word out per step where the buffers
 // allow it (a float a thread with single-byte stores took 17.7 us for
 // 1920x1080 RGBA, 2.3 TB/s), two steps in flight.
-__global__ void __launch_bounds__(256) quantize4_kernel(const float *__restrict__ in, uint8_t *__restrict__ out,
-                                                        long long n)
+__global__ void __launch_bounds__(256) quantize4_kernel(const float4 *__restrict__ in, uchar4 *__restrict__ out,
+                                                        long long n4, int rest)
 {
-    const float4 *in4 = reinterpret_cast<const float4 *>(in);
-    uchar4 *out4 = reinterpret_cast<uchar4 *>(out);
-    const long long stride = (long long) gridDim.x * blockDim.x, n4 = n / 4;
-    const long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
-    for (long long i = t; i < n4; i += 2 * stride) {
+    const long long stride = (long long) gridDim.x * blockDim.x;
+    for (long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n4; i += 2 * stride) {
         const bool two = i + stride < n4;
-        const float4 a = __ldg(in4 + i), b = two ? __ldg(in4 + i + stride) : a;
-        out4[i] = make_uchar4(q8k(a.x), q8k(a.y), q8k(a.z), q8k(a.w));
-        if (two) out4[i + stride] = make_uchar4(q8k(b.x), q8k(b.y), q8k(b.z), q8k(b.w));
+        const float4 a = __ldg(in + i), b = two ? __ldg(in + i + stride) : a;
+        out[i] = make_uchar4(q8k(a.x), q8k(a.y), q8k(a.z), q8k(a.w));
+        if (two) out[i + stride] = make_uchar4(q8k(b.x), q8k(b.y), q8k(b.z), q8k(b.w));
     }
-    if (t < n - 4 * n4) out[4 * n4 + t] = (uint8_t) q8k(in[4 * n4 + t]);
+    if (blockIdx.x == 0 && threadIdx.x < rest)  // the last n % 4 floats
+        reinterpret_cast<uint8_t *>(out + n4)[threadIdx.x] =
+            (uint8_t) q8k(reinterpret_cast<const float *>(in + n4)[threadIdx.x]);
 }
 
 // unaligned buffers
@@ -990,7 +989,9 @@ cudaError_t launch_composite(float *dst, const float *src, int num, long long np
 cudaError_t launch_quantize(const float *in, uint8_t *out, long long n, cudaStream_t s)
 {
     const bool vec = reinterpret_cast<uintptr_t>(in) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 4 == 0;
-    if (vec) quantize4_kernel<<<grid_for((n + 3) / 4, 256), 256, 0, s>>>(in, out, n);
+    if (vec)
+        quantize4_kernel<<<grid_for((n + 3) / 4, 256), 256, 0, s>>>((const float4 *) in, (uchar4 *) out, n / 4,
+                                                                     (int) (n % 4));
     else quantize_kernel<<<grid_for(n, 256), 256, 0, s>>>(in, out, n);
     return cudaGetLastError();
 }
