@@ -59,11 +59,27 @@ PROFILES = os.path.join(ROOT, "profiles")
 # committed ncu summaries carrying dram_bytes_per_launch of the dominant kernel
 PROFILE_TRAFFIC = {"learned_1024": os.path.join(PROFILES, "march_judged_learned_1024.txt"),
                    "sorted_brick_512": os.path.join(PROFILES, "march_cfg_sorted_brick_512.txt")}
-# kernel launches of one frame: learned skipping = tile cost + tile scatter
-# + judged march + judge compare + gated exact re-march; the exact grid =
-# tile cost + tile scatter + march
-LAUNCHES_LEARNED = 5
-LAUNCHES_GRID = 3
+# kernel launches of one frame: learned skipping = judged march + judge compare
+# + gated exact re-march; else the march.  Where the cost order of the tiles is
+# asked for, tile cost and tile scatter before it, in frames of at least 8 tiles
+# (8x4 pixels) a resident warp (5 blocks of 4 warps an SM)
+LAUNCHES_LEARNED = 3
+LAUNCHES_ORDER = 2
+ORDER_TILES_PER_SM = 8 * 5 * 4
+
+
+def frame_launches(skip, tiles, w, h, sms):
+    """Kernel launches of a w x h CONFIG frame with the given skip mode and tile
+    order ("cost" or "raster") on a GPU of so many SMs."""
+    from ivr_gb300 import api
+    n = LAUNCHES_LEARNED if skip == api.SKIP_LEARNED else 1
+    ordered = tiles == "cost" and skip != api.SKIP_NONE
+    return n + (LAUNCHES_ORDER if ordered and (w + 7) // 8 * ((h + 3) // 4) >= ORDER_TILES_PER_SM * sms else 0)
+
+
+def sm_count():
+    import torch
+    return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
 
 
 class ClockSampler:
@@ -632,9 +648,7 @@ def run_learned(args, quiet=False):
             "judge_timed_frames": judge_timed,
             "methods": methods,
             "training": training, "ingest": ingest,
-            "gpu_launches": args.steps * ((LAUNCHES_LEARNED if skip == api.SKIP_LEARNED else
-                                           LAUNCHES_GRID if skip == api.SKIP_GRID else 1)
-                                          - (2 if args.tiles == "raster" and skip != api.SKIP_NONE else 0)),
+            "gpu_launches": args.steps * frame_launches(skip, args.tiles, w, h, sm_count()),
             "clocks": clk.summary(),
         }
         if not args.no_cpu_baseline and world == 1:
@@ -955,7 +969,7 @@ def run_sorted(args, quiet=False, name="sorted_brick_512"):
                                      "filtered-texture peak = one hardware-filtered 3D-texture fetch per sample "
                                      "(the hardware trilinear ceiling); hbm = compulsory bytes (the macrocells an "
                                      "executed sample read + RGBA8 out) over the frame time"},
-            "gpu_launches": args.steps * (LAUNCHES_GRID if args.tiles == "cost" else 1),
+            "gpu_launches": args.steps * frame_launches(api.SKIP_GRID, args.tiles, w, h, sm_count()),
             "clocks": clk.summary(),
         }
         if other_cells:
