@@ -485,11 +485,26 @@ int ivr_mlp_train(ivr_mlp *m, int epochs, int batch_rows, float lr, float wneg, 
     if (rc) return rc;
     // Workspaces of the epochs, kept with the predictor.  On the device: the
     // Adam bias corrections of an epoch's steps, so that one captured epoch
-    // replays with each epoch's values.  Page-locked, in one block: the epochs'
+    // replays with each epoch's values (under a budget they are given back, for
+    // what follows the training may need the room).  Page-locked, in one block: the epochs'
     // row orders (the host shuffles the next epoch's while the device trains
     // on the current one; one buffer if there is no next), the epoch's bias
     // corrections and its losses, so that no copy of an epoch waits for the
     // host or the host for the device before the shuffle is done.
+    struct Corrections {
+        ivr_mlp *m;
+        void release()
+        {
+            dev_free(m->ctx, m->d_c12, (size_t) m->c12_cap * sizeof(float));
+            m->d_c12 = nullptr;
+            m->c12_cap = 0;
+        }
+        ~Corrections()
+        {
+            if (m->ctx->budget) release();
+        }
+    } corrections{m};
+    if (m->c12_cap < 2 * nb) corrections.release();
     rc = grow(c, (void **) &m->d_c12, &m->c12_cap, 2 * nb, sizeof(float), 0);
     if (rc) return rc;
     const size_t n = (size_t) m->n;
