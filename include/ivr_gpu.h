@@ -138,6 +138,12 @@ void ivr_params_config(ivr_render_params *p);  /* CONFIG defaults */
 int ivr_create(int device, size_t hbm_budget_bytes, ivr_ctx **out); /* budget 0 = no limit */
 int ivr_destroy(ivr_ctx *ctx);
 const char *ivr_last_error(const ivr_ctx *ctx);
+/* Device bytes of the arrays that the context's objects use: what the budget is
+ * held against.  The device gives somewhat more: arrays that share an allocation
+ * start on 512 bytes, and without a budget a volume holds the allocation of its
+ * corner-packed copies for its next brick layout, three slabs of the volume's
+ * copy larger than its largest layout's copies so far (until ivr_volume_free or
+ * ivr_volume_set_quads(volume, 0)). */
 int ivr_mem_used(const ivr_ctx *ctx, size_t *bytes);
 
 /* Device memory counted against the context's HBM budget (for callers'
