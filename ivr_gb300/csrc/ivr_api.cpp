@@ -92,8 +92,9 @@ struct BlockArray {
 // The driver takes some 30 us to allocate an array, 30 to free one, and 0.3 and
 // 0.5 us a megabyte more.  Eight bricks have 24 arrays, their skipping grid 17:
 // arrays that live and die together are parts of one block (384^3 f32 volume,
-// 2x2x2 bricks, opened up to its first frame: 5.2 -> 4.8 ms, and 3.8 with the
-// corner-packed copies' block kept from layout to layout).
+// 2x2x2 bricks, opened up to its first frame: 5.2 -> 4.8 ms, and 3.7 with the
+// corner-packed copies' block kept from layout to layout; what the driver takes
+// differs from box to box, on another one the same three steps were 5.9 -> 5.0).
 constexpr size_t kBlockAlign = 512;
 
 size_t block_bytes(const std::vector<BlockArray> &arrays)

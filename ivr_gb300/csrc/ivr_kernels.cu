@@ -598,9 +598,10 @@ __device__ __forceinline__ unsigned q8k(float v)
     return (unsigned) ((255ull * m + (1ull << (s - 1))) >> s);
 }
 
-// HBM-bound; four floats in, one 32-bit word out per step where the buffers
-// allow it (a float a thread with single-byte stores took 17.7 us for
-// 1920x1080 RGBA, 2.3 TB/s), two steps in flight.
+// Four floats in, one 32-bit word out per step where the buffers allow it, two
+// steps in flight.  Bound by HBM and by q8k's 64-bit integers, each about half:
+// 1920x1080 RGBA in 12.4 us (3.3 TB/s, issue slots 66% full); a float a thread
+// with single-byte stores took 17.7.
 __global__ void __launch_bounds__(256) quantize4_kernel(const float4 *__restrict__ in, uchar4 *__restrict__ out,
                                                         long long n4, int rest)
 {
