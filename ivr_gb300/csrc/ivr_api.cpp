@@ -94,7 +94,7 @@ struct BlockArray {
 // arrays that live and die together are parts of one block (384^3 f32 volume,
 // 2x2x2 bricks, opened up to its first frame: 5.2 -> 4.8 ms, and 3.7 with the
 // corner-packed copies' block kept from layout to layout; what the driver takes
-// differs from box to box, on another one the same three steps were 5.9 -> 5.0).
+// differs from machine to machine: 5.9 -> 5.0 in all on another one).
 constexpr size_t kBlockAlign = 512;
 
 size_t block_bytes(const std::vector<BlockArray> &arrays)
